@@ -204,6 +204,7 @@ hm_status layout(hm_batch *b, int groups) {
         const double b2 = p.barrier * p.barrier;
         sd[q].b2bits = 0;
         if (!std::isnan(b2)) std::memcpy(&sd[q].b2bits, &b2, sizeof(b2));
+        sd[q].pair_hi = hm::pair_threshold_hi(b2, p.mu);
         std::fill(set_of.begin() + b->offsets[k], set_of.begin() + b->offsets[k + 1], uint32_t(q));
     }
     // Tile-table capacity of each group: one warp-tile per 32 particles at

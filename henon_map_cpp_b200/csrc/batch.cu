@@ -148,7 +148,7 @@ __device__ __forceinline__ void run_tile(const BatchDev &b, const BatchSetDev &s
     }
     const uint32_t turn0 = st.done, nt = st.turns;
     const double mu = set.mu;
-    // The common path needs only the coordinate bound of the barrier test;
+    // The common path needs only the coordinate bounds of the barrier test;
     // the rare per-turn redo rebuilds the whole test from b2bits.
     const uint32_t small_hi = dev::make_barrier<ARITH>(set.b2bits).small_hi;
     bool warp_live = __any_sync(dev::kFullMask, any);
@@ -165,30 +165,26 @@ __device__ __forceinline__ void run_tile(const BatchDev &b, const BatchSetDev &s
             stage_async(bufs + ((sg + 1u) & 1u) * kStageTurns * 4u, set.table,
                         turn0 + k0 + kStageTurns, min(kStageTurns, nt - k0 - kStageTurns), lane);
         const double *rec = bufs + (sg & 1u) * kStageTurns * 4u;
-        // The stage's turns with no per-turn control flow, ORing every
-        // coordinate's high word; one vote at the end.  Only a warp with a
-        // coordinate at or above the bound of dev::small_or restores the
-        // saved particles and redoes the stage with the per-turn test
-        // (the scheme of the tracking kernel, track.cu turns_staged).
+        // The stage's turns with no per-turn control flow (dev::block_turns);
+        // one vote at the end.  Only a warp with a coordinate at or above the
+        // bound restores the saved particles and redoes the stage with the
+        // per-turn test (the scheme of the tracking kernel, track.cu
+        // turns_staged).
 #pragma unroll
         for (int j = 0; j < K; ++j) {
             ckpt[2 * (j * 32 + int(lane))] = make_double2(p[j].x, p[j].px);
             ckpt[2 * (j * 32 + int(lane)) + 1] = make_double2(p[j].y, p[j].py);
         }
-        uint32_t ored_stage = 0u;
-        for (uint32_t kk = 0; kk < kn_stage; ++kk) {
-            const double2 *q = reinterpret_cast<const double2 *>(rec + 4u * kk);
-            const double2 q0 = q[0], q1 = q[1];
-            const dev::Turn t{q0.x, q0.y, q1.x, q1.y};
-#pragma unroll
-            for (int j = 0; j < K; ++j) {
-                dev::turn<ARITH, OCT, false>(p[j], t, mu);
-                ored_stage |= dev::hi_or(p[j]);
-            }
+        const double2 *const q0 = reinterpret_cast<const double2 *>(rec);
+        bool over = false;
+        if (kn_stage == kStageTurns) {
+#pragma unroll 1
+            for (uint32_t kk = 0; kk < kStageTurns; kk += dev::kBlockTurns)
+                over |= dev::block_turns<ARITH, OCT, false, K>(p, q0 + 2u * kk, mu) >= set.pair_hi;
+        } else {
+            over = dev::each_turn<ARITH, OCT, false, K>(p, q0, kn_stage, mu) >= small_hi;
         }
-        // (small_or with the bound alone: the OR of the high words, sign
-        // masked, against the coordinate bound)
-        const bool redo = __any_sync(dev::kFullMask, (ored_stage & 0x7fffffffu) >= small_hi);
+        const bool redo = __any_sync(dev::kFullMask, over);
         if (redo) {
 #pragma unroll
             for (int j = 0; j < K; ++j) {
@@ -267,13 +263,15 @@ __device__ __forceinline__ void run_tile(const BatchDev &b, const BatchSetDev &s
     }
 }
 
-// Persistent: warps pop warp-tiles until the chunk's queue is empty.  With
-// the turn records copied by cp.async (no staging registers), particle
-// slots recomputed from the tile and only the barrier's coordinate bound in
-// registers, one particle per thread fits 64 registers (8 blocks per SM)
-// and two fit 90 (5 blocks per SM).
+// Persistent: warps pop warp-tiles until the chunk's queue is empty.  One
+// particle per thread may use 128 registers (4 blocks per SM): as in the
+// tracking kernel, loading the next turns' records ahead is worth more than
+// more warps.  64 mixed sets of 1e3 to 6.4e4 particles, 1e3 to 2e5 turns:
+// 25.0 ms against 28.3 with 64 registers (8 blocks), fast arithmetic 18.9
+// against 22.9; with 1e3 to 2.56e5 particles and 3e5 turns 83.3 against
+// 84.6 and 61.0 against 62.8.
 template <int ARITH, int K>
-__global__ void __launch_bounds__(kThreads, K == 1 ? 8 : (K == 2 ? 5 : 1))
+__global__ void __launch_bounds__(kThreads, K == 1 ? 4 : (K == 2 ? 5 : 1))
     batch_chunk_kernel(BatchDev b) {
     __shared__ __align__(16) double stage_bufs[kWarps][2 * kStageTurns * 4];
     // Per warp, the particles {x, px}, {y, py} at the start of a stage.

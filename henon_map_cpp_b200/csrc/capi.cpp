@@ -23,13 +23,17 @@ std::atomic<void *> g_cancel_ctx{nullptr};
 // Launch shape of the tracking kernels (set by the autotuner).
 struct TrackConfig {
     int threads = 128;
-    int per_thread = 2;
+    // One particle per thread: a redo (track.cu turns_staged) repeats the
+    // turns of 32 particles instead of 64, and short lists balance better.
+    // 1024^2 grid on [0, 0.6]^2, mu = 0.2, 2e4 turns: 28.0 ms against 29.6
+    // with two; fast arithmetic, 701^2, mu = 0: 7.45 against 7.69.
+    int per_thread = 1;
     uint32_t chunk0 = 512;      // turns of the first chunk
     uint32_t chunk_max = 16384; // chunk length cap (chunks double up to it)
     // Turn records per staged bulk copy (0: direct reads).  Staging measured
-    // 2-4 % faster than direct reads on the DA scan (1024^2 grid, 1e5 turns:
-    // 17.7 vs 17.1 FP64 TFLOP/s at 256 turns a stage).
-    uint32_t stage_turns = 256;
+    // 2-4 % faster than direct reads on the DA scan, stages of 512 turns 1 %
+    // faster than 256 (two particles per thread: 29.6 and 29.9 ms).
+    uint32_t stage_turns = 512;
 };
 std::mutex g_cfg_mutex;
 TrackConfig g_cfg;
@@ -292,7 +296,8 @@ hm_status track_driver(double *x, double *px, double *y, double *py,
                        uint64_t table_len, uint32_t s0, uint32_t n_turns,
                        double mu, double barrier, bool inverse, hm_arith arith,
                        void *workspace, cudaStream_t stream,
-                       uint32_t *turns_done, double kick_module, unsigned long long kick_seed) {
+                       uint32_t *turns_done, double kick_module, unsigned long long kick_seed,
+                       bool own_table) {
     *turns_done = 0;
     if (n == 0 || n_turns == 0) {
         *turns_done = n_turns;  // nothing to move; the turn counter still advances
@@ -326,6 +331,8 @@ hm_status track_driver(double *x, double *px, double *y, double *py,
     c.b2bits = b2bits;
     c.kick_module = kick_module;
     c.kick_seed = kick_seed;
+    c.pair_hi = pair_threshold_hi(b2, mu);
+    c.check_records = !own_table;
     TrackLaunch l{int(arith), mu != 0.0, inverse, cfg.per_thread, cfg.threads};
 
     const bool one_chunk = n_turns <= cfg.chunk0;
@@ -333,11 +340,17 @@ hm_status track_driver(double *x, double *px, double *y, double *py,
         return fail(HM_ERR_INVALID_ARG, "workspace required for more than one chunk of turns");
     Workspace w{};
     if (!one_chunk) w = carve(workspace, n);
-    // Staged turn records need the workspace's fault word and a table that
-    // bulk copies can read (16-byte aligned).
-    const bool staged = cfg.stage_turns != 0 && !one_chunk &&
-                        (reinterpret_cast<uintptr_t>(table) & 15u) == 0;
+    // Staged turn records need a table that double2 loads and bulk copies can
+    // read (16-byte aligned), and the bulk copies the workspace's fault word.
+    // A call of one chunk stages all its records at once, without bulk
+    // copies; below 16 turns the direct reads are as quick.
+    const bool stageable = cfg.stage_turns != 0 && (reinterpret_cast<uintptr_t>(table) & 15u) == 0;
+    const bool staged = stageable && !one_chunk;
     c.stage_turns = staged ? cfg.stage_turns : 0u;
+    if (stageable && one_chunk && n_turns >= 16u && n_turns <= 512u) {
+        c.stage_turns = 16u;
+        while (c.stage_turns < n_turns) c.stage_turns *= 2u;
+    }
     c.fault = staged ? w.fault : nullptr;
     if (staged) HM_CUDA_TRY(cudaMemsetAsync(w.fault, 0, sizeof(uint32_t), stream));
 
@@ -385,6 +398,14 @@ hm_status track_driver(double *x, double *px, double *y, double *py,
         done += len;
         chunk = std::min<uint32_t>(chunk * 2u, cfg.chunk_max);
         if (last) break;
+        // The short chunks are enqueued without waiting for their survivor
+        // counts: the next grid covers the last count known, and its blocks
+        // past the list end at once.  A wait costs about 15 us, as much as
+        // 500 turns of a small set.
+        if (len < cfg.chunk_max && !timer.armed) {
+            cur = nxt;
+            continue;
+        }
         uint32_t counters[3];  // count[0], count[1], fault
         HM_CUDA_TRY(cudaMemcpyAsync(counters, w.count[0], sizeof(counters),
                                     cudaMemcpyDeviceToHost, stream));
@@ -935,7 +956,7 @@ hm_status hm_track(hm_tracker *t, hm_particles *p, uint32_t n_turns, double mu, 
         p->x.as<double>(), p->px.as<double>(), p->y.as<double>(), p->py.as<double>(),
         p->steps.as<uint32_t>(), p->n_total, t->table.as<const double>(), t->allowed_steps,
         p->live_step, n_turns, mu, barrier, inverse != 0, t->arith, ws, 0, &done, kick_module,
-        p->kick_seed);
+        p->kick_seed, true);
     if (s != HM_OK && s != HM_ERR_CANCELLED) return s;
     // global_steps follows the turns applied (src/henon.cu:3181-3184).
     if (inverse) {

@@ -393,6 +393,89 @@ __device__ __forceinline__ bool small_or(uint32_t ored, const Barrier &b) {
     return (ored & 0x7fffffffu) < b.small_hi;
 }
 
+// The largest |high word| of a and b and of the running maximum m, taken on
+// the words read as single floats: for sign-free patterns both orders agree,
+// and a pattern at or above 0x7f800000 (a coordinate of 2^1016 or more, an
+// infinity or a NaN) gives infinity or, with .NaN, a NaN, whose pattern is
+// above every bound.  One instruction for two coordinates.
+__device__ __forceinline__ float hi_max(float m, double a, double b) {
+    float r;
+    asm("max.NaN.abs.f32 %0, %1, %2, %3;"
+        : "=f"(r)
+        : "f"(m), "f"(__int_as_float(__double2hiint(a))), "f"(__int_as_float(__double2hiint(b))));
+    return r;
+}
+
+// A block of kBlockTurns turns with no per-turn control flow: the turns are
+// applied, the largest high word of the coordinates after every second turn
+// is kept, and the caller votes once per block.  Records are read from q,
+// one {sx, cx}, {sy, cy} pair of double2 per turn, forwards or (REV)
+// backwards.
+//
+// Why every second turn is enough: a turn is a rotation of each plane and a
+// kick of the momenta by (x^2 - y^2, -2xy) and, with the octupole,
+// mu (x^3 - 3xy^2, y^3 - 3x^2y), whose lengths are |z|^2 and |mu| |z|^3,
+// z = (x, y).  So with R the length of the state after a turn, forward or
+// backward, the state before it is at most g(R) = R + R^2 + |mu| R^3 long.
+// If every coordinate after the second turn of a pair is below t with g(2t)
+// below the barrier, both turns were inside; the caller compares with the
+// high word of that t (pair_threshold_hi, hm_internal.h, where the rounding
+// errors are covered).  It needs records that are rotations
+// (sx^2 + cx^2 = 1), which the library's own tables are; a caller's table
+// is checked first.
+//
+// Cycles per warp and turn (exact, mu = 0, one particle per thread, 32 warps
+// per SM; the 19 FP64 instructions take two each, 38): 39.2 without any
+// look, 44.5 looking at every turn (the two three-input instructions of a
+// look read FP64 results and cost about 2.5 cycles each, more than their
+// slots), 41.7 at every second.  Unrolled, the loads of the next turns'
+// records issue early: 50 instead of 63 cycles (unrolled by 2) with one warp
+// per scheduler.
+constexpr uint32_t kBlockTurns = 16u;
+
+// Returns the pattern to compare with the bound (below it: nothing lost).
+template <int ARITH, bool OCT, bool REV, int K>
+__device__ __forceinline__ uint32_t block_turns(Particle (&p)[K], const double2 *q, double mu) {
+    constexpr int D = REV ? -2 : 2;
+    constexpr int kUnroll = K <= 2 ? int(kBlockTurns) : 4;
+    float big = 0.0f;
+#pragma unroll kUnroll
+    for (int u = 0; u < int(kBlockTurns); ++u) {
+        const double2 a = q[u * D], b = q[u * D + 1];
+#pragma unroll
+        for (int j = 0; j < K; ++j) {
+            turn<ARITH, OCT, REV>(p[j], Turn{a.x, a.y, b.x, b.y}, mu);
+            if (u & 1) big = hi_max(hi_max(big, p[j].x, p[j].px), p[j].y, p[j].py);
+        }
+    }
+    return __float_as_uint(big) & 0x7fffffffu;
+}
+
+// n turns, every one looked at (a short block, or records that are not
+// rotations): the bound is Barrier::small_hi.
+template <int ARITH, bool OCT, bool REV, int K>
+__device__ __forceinline__ uint32_t each_turn(Particle (&p)[K], const double2 *q, uint32_t n,
+                                              double mu) {
+    constexpr int D = REV ? -2 : 2;
+    float big = 0.0f;
+#pragma unroll 1
+    for (uint32_t k = 0; k < n; ++k, q += D) {
+        const double2 a = q[0], b = q[1];
+#pragma unroll
+        for (int j = 0; j < K; ++j) {
+            turn<ARITH, OCT, REV>(p[j], Turn{a.x, a.y, b.x, b.y}, mu);
+            big = hi_max(hi_max(big, p[j].x, p[j].px), p[j].y, p[j].py);
+        }
+    }
+    return __float_as_uint(big) & 0x7fffffffu;
+}
+
+// sx^2 + cx^2 and sy^2 + cy^2 within 2^-12 of 1 (false for NaN).
+__device__ __forceinline__ bool is_rotation(double2 a, double2 b) {
+    return fabs(fma(a.x, a.x, fma(a.y, a.y, -1.0))) < 0x1p-12 &&
+           fabs(fma(b.x, b.x, fma(b.y, b.y, -1.0))) < 0x1p-12;
+}
+
 // Every coordinate is small (no FP64 instruction).
 __device__ __forceinline__ bool small_inside(const Particle &p, const Barrier &b) {
     const uint32_t m = max(max(abs_hi(p.x), abs_hi(p.px)), max(abs_hi(p.y), abs_hi(p.py)));

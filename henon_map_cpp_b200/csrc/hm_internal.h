@@ -1,8 +1,10 @@
 // Internal declarations shared by the host side of libhenon_b200.so.
 #pragma once
 
+#include <cmath>
 #include <cstddef>
 #include <cstdint>
+#include <cstring>
 #include <mutex>
 #include <random>
 #include <string>
@@ -135,6 +137,35 @@ namespace hm {
 
 // ---- kernel launchers (defined in the .cu files) ---------------------------
 
+// High word of the largest coordinate bound t for which a state with all
+// |coordinates| < t cannot be one turn past a state outside the barrier
+// (dev::run_turns): g(2t) = R + R^2 + |mu| R^3 < barrier at R = 2t.  R is
+// found from above by Newton's method (g is convex and increasing, so the
+// iterates stay above the root) and then shrunk until g(R) is below the
+// barrier less 2^-8 of it.  That margin covers the roundings of a turn (a
+// few units of 2^-53 of each term, and absolute errors of 2^-1075 where a
+// product is subnormal, excluded by barrier^2 >= 2^-900) and the 2^-12 by
+// which a checked record may miss a rotation.  0 (no state passes) for a
+// NaN or tiny barrier and for a NaN or infinite mu.
+inline uint32_t pair_threshold_hi(double barrier2, double mu) {
+    const double r2 = std::fmin(barrier2, 1.7976931348623157e308);
+    const double m = std::fabs(mu);
+    if (!(barrier2 >= 0x1p-900) || !(m <= 1.7976931348623157e308)) return 0u;
+    const double b = std::sqrt(r2) * (1.0 - 0x1p-8);
+    double R = std::fmin(b, std::sqrt(b));
+    if (m > 0.0) R = std::fmin(R, std::cbrt(b / m));
+    auto g = [m](double r) { return r + r * r + m * r * r * r; };
+    for (int it = 0; it < 16; ++it)
+        R -= (g(R) - b) / (1.0 + 2.0 * R + 3.0 * m * R * R);
+    for (int it = 0; it < 64 && !(g(R) < b); ++it) R *= 1.0 - 0x1p-10;
+    if (!(g(R) < b) || !(R > 0.0)) return 0u;
+    const double t = R * 0.5 * (1.0 - 0x1p-20);
+    uint64_t bits;
+    std::memcpy(&bits, &t, sizeof(bits));
+    return uint32_t(bits >> 32);
+}
+
+
 // Parameters of one fused multi-turn chunk launch over a list of particles.
 struct TrackChunk {
     // Caller state, indexed by the original particle index.
@@ -163,6 +194,11 @@ struct TrackChunk {
     // (a power of two in [16, 512]; needs a 16-byte aligned table).
     uint32_t stage_turns;
     uint32_t *fault;       // set to nonzero when a staged copy timed out
+    // High word of the coordinate bound of the test that looks at every
+    // second turn (pair_threshold_hi; 0 disables it), and whether the
+    // records have to be checked to be rotations first (a caller's table).
+    uint32_t pair_hi;
+    bool check_records;
     // Random kick of this module per turn (NaN: none), direction keyed by
     // (kick_seed, caller's particle index, table index of the turn).
     double kick_module;
@@ -199,7 +235,7 @@ hm_status track_driver(double *x, double *px, double *y, double *py,
                        double mu, double barrier, bool inverse, hm_arith arith,
                        void *workspace, cudaStream_t stream,
                        uint32_t *turns_done, double kick_module = __builtin_nan(""),
-                       unsigned long long kick_seed = 0ull);
+                       unsigned long long kick_seed = 0ull, bool own_table = false);
 
 // Elementwise observable kernel launcher.
 cudaError_t launch_observable(const double *x, const double *px,
@@ -300,6 +336,7 @@ struct BatchSetDev {
     uint32_t n_turns;      // turn budget
     double mu;
     long long b2bits;      // bit pattern of barrier^2 (0 when NaN)
+    uint32_t pair_hi;      // pair_threshold_hi(barrier^2, mu)
 };
 
 struct BatchStateDev {

@@ -99,14 +99,11 @@ __device__ __forceinline__ void turns_direct(const TrackChunk &c, const Barrier 
     }
 }
 
-// Turns between two barrier votes of the staged kernel (see turns_staged).
-constexpr uint32_t kCheckTurns = 32;
-
 // Shared memory of a staged launch: two stage buffers of turn records and,
-// without kicks, one checkpoint {x, px, y, py} per particle.
+// without kicks, two checkpoints {x, px, y, py} per particle.
 __host__ __device__ constexpr size_t staged_smem_bytes(uint32_t stage_turns, uint32_t threads,
                                                        int per_thread, bool kick) {
-    return size_t(stage_turns) * 2u * 32u + (kick ? 0u : size_t(threads) * per_thread * 32u);
+    return size_t(stage_turns) * 2u * 32u + (kick ? 0u : size_t(threads) * per_thread * 64u);
 }
 
 __device__ __forceinline__ Turn staged_record(const double *rec, uint32_t kn, uint32_t kk,
@@ -124,16 +121,19 @@ __device__ __forceinline__ Turn staged_record(const double *rec, uint32_t kn, ui
 // broadcast.  Warps whose particles are all lost keep taking part in the
 // per-stage barriers; the block stops when none of its warps is live.
 //
-// Without kicks, a stage runs in runs of kCheckTurns turns with no
-// per-turn control flow: the thread saves its particles to shared memory,
-// applies the turns while ORing every coordinate's high word, and the warp
-// votes once at the end.  If no coordinate of any turn reached the bound
-// of dev::small_or, no particle can have been lost in the run, which is
-// then exactly what the per-turn test would have produced.  Otherwise the
-// warp restores the saved particles and redoes the run with the per-turn
-// test (turn_all), which finds the loss turn.  A per-turn vote made each
-// turn wait for the tail of the previous one; a redo costs one run per
-// loss event of a warp.
+// Without kicks, a stage runs in blocks of turns with no per-turn control
+// flow (dev::block_turns): the thread saves its particles to shared memory
+// and applies the block's turns.  If the coordinates looked at stayed below
+// the bound, no particle can have been lost in the block, which is then
+// exactly what the per-turn test would have produced.  Otherwise the warp
+// restores the saved particles and redoes the block with the per-turn test
+// (turn_all).  The warp votes on a block while it already runs the next one
+// (hence two checkpoints): a vote before each block made every warp wait
+// for the end of its chain of turns, 54 instead of 50 cycles a turn with one
+// warp per scheduler and 43.9 instead of 43.2 with four.  Sixteen turns keep
+// a loss cheap (at most 32 turns repeated) where a fifth of the particles is
+// lost in 512 turns; blocks of 8 cost 1.4 cycles a turn more and runs of 128
+// turns 4 % of the dynamic-aperture scan.
 // Returns false when a copy did not land within the bounded wait (the
 // chunk's results are then invalid and c.fault is set).
 template <int ARITH, bool OCT, bool REV, int K, bool KICK>
@@ -155,13 +155,21 @@ __device__ __forceinline__ bool turns_staged(const TrackChunk &c, const Barrier 
         dev::bulk_load(stage_buf + size_t(st & 1u) * S * 4u, c.table + size_t(lo) * 4u,
                        kn * 32u, &full[st & 1u]);
     };
-    if (leader) {
+    // A chunk of one stage has nothing to overlap: the block copies its
+    // records itself, and no copy can time out.
+    const bool one_stage = n_stages == 1;
+    if (one_stage) {
+        const double2 *const src = reinterpret_cast<const double2 *>(
+            c.table + size_t(REV ? c.turn0 - nt : c.turn0) * 4u);
+        double2 *const dst = reinterpret_cast<double2 *>(stage_buf);
+        for (uint32_t i = threadIdx.x; i < 2u * nt; i += blockDim.x) dst[i] = __ldg(src + i);
+    } else if (leader) {
         dev::mbar_init(&full[0], 1);
         dev::mbar_init(&full[1], 1);
         dev::mbar_init_fence();
     }
     __syncthreads();
-    if (leader) {
+    if (leader && !one_stage) {
         if (n_stages > 0) issue(0);
         if (n_stages > 1) issue(1);
     }
@@ -170,7 +178,7 @@ __device__ __forceinline__ bool turns_staged(const TrackChunk &c, const Barrier 
     for (; st < n_stages; ++st) {
         const uint32_t buf = st & 1u;
         // Warp-uniform, so that the turn loop's warp votes see every lane.
-        const bool landed = dev::mbar_wait(&full[buf], (st >> 1) & 1u);
+        const bool landed = one_stage || dev::mbar_wait(&full[buf], (st >> 1) & 1u);
         if (!__all_sync(kFullMask, landed)) timed_out = true;
         const uint32_t k0 = st * S;
         const uint32_t kn = min(S, nt - k0);
@@ -181,34 +189,75 @@ __device__ __forceinline__ bool turns_staged(const TrackChunk &c, const Barrier 
                 turn_all<ARITH, OCT, REV, K, KICK>(c, bar, mu, staged_record(rec, kn, kk, REV),
                                                    k0 + kk, p, id, live, warp_live);
         } else if (!timed_out) {
-            for (uint32_t j0 = 0; warp_live && j0 < kn; j0 += kCheckTurns) {
-                const uint32_t j1 = min(j0 + kCheckTurns, kn);
+            // A caller's records are checked to be rotations, which the
+            // test of every second turn needs.
+            bool pairs = c.pair_hi != 0u;
+            if (pairs && c.check_records) {
+                const double2 *q = reinterpret_cast<const double2 *>(rec);
+                bool unit = true;
+                for (uint32_t kk = threadIdx.x & 31u; kk < kn; kk += 32u)
+                    unit = unit && dev::is_rotation(q[2u * kk], q[2u * kk + 1u]);
+                pairs = __all_sync(kFullMask, unit);
+            }
+            constexpr uint32_t B = dev::kBlockTurns;
+            const uint32_t pair_hi = c.pair_hi;
+            const double2 *const q0 =
+                reinterpret_cast<const double2 *>(rec) + (REV ? 2u * (kn - 1u) : 0u);
+            auto record = [&](uint32_t kk) { return REV ? q0 - 2u * kk : q0 + 2u * kk; };
+            double2 *save = ckpt, *saved = ckpt + size_t(2u * K) * blockDim.x;
+            auto checkpoint = [&]() {
 #pragma unroll
                 for (int j = 0; j < K; ++j) {
-                    ckpt[2u * (j * blockDim.x + threadIdx.x)] = make_double2(p[j].x, p[j].px);
-                    ckpt[2u * (j * blockDim.x + threadIdx.x) + 1u] = make_double2(p[j].y, p[j].py);
+                    double2 *const to = save + 2u * (j * blockDim.x + threadIdx.x);
+                    to[0] = make_double2(p[j].x, p[j].px);
+                    to[1] = make_double2(p[j].y, p[j].py);
                 }
-                uint32_t ored = 0u;
+            };
+            auto swap = [&]() {
+                double2 *const t = save;
+                save = saved;
+                saved = t;
+            };
+            bool check = false;  // this thread's verdict on the block before
+            for (uint32_t j0 = 0; warp_live && j0 < kn;) {
+                bool again = false;  // the warp's
+                // The hot loop holds nothing but blocks: with the redo's code
+                // inside it a turn took 3 cycles more.
+                const uint32_t jb = pairs ? j0 + (kn - j0) / B * B : j0;
+                const double2 *q = record(j0);
 #pragma unroll 2
-                for (uint32_t kk = j0; kk < j1; ++kk) {
-                    const Turn t = staged_record(rec, kn, kk, REV);
-#pragma unroll
-                    for (int j = 0; j < K; ++j) {
-                        dev::turn<ARITH, OCT, REV>(p[j], t, mu);
-                        ored |= dev::hi_or(p[j]);
+                for (; j0 < jb; j0 += B, q += REV ? -int(2u * B) : int(2u * B)) {
+                    checkpoint();
+                    again = __any_sync(kFullMask, check);
+                    const bool next = dev::block_turns<ARITH, OCT, REV, K>(p, q, mu) >= pair_hi;
+                    if (again) break;
+                    check = next;
+                    swap();
+                }
+                if (!again && j0 < kn) {  // a short block, or records of another kind
+                    checkpoint();
+                    again = __any_sync(kFullMask, check);
+                    if (!again) {
+                        check = dev::each_turn<ARITH, OCT, REV, K>(p, record(j0), min(B, kn - j0),
+                                                                   mu) >= bar.small_hi;
+                        j0 += B;
+                        swap();
                     }
                 }
-                if (__any_sync(kFullMask, !dev::small_or(ored, bar))) {
+                if (!again && j0 >= kn) again = __any_sync(kFullMask, check);
+                if (again) {  // the block that ended at j0, turn by turn
 #pragma unroll
                     for (int j = 0; j < K; ++j) {
-                        const double2 a = ckpt[2u * (j * blockDim.x + threadIdx.x)];
-                        const double2 b = ckpt[2u * (j * blockDim.x + threadIdx.x) + 1u];
+                        const double2 *const from = saved + 2u * (j * blockDim.x + threadIdx.x);
+                        const double2 a = from[0], b = from[1];
                         p[j] = dev::make_particle(a.x, a.y, b.x, b.y);
                     }
-                    for (uint32_t kk = j0; warp_live && kk < j1; ++kk)
+                    const uint32_t j1 = min(j0, kn);
+                    for (uint32_t kk = j0 - B; warp_live && kk < j1; ++kk)
                         turn_all<ARITH, OCT, REV, K, KICK>(c, bar, mu,
-                                                           staged_record(rec, kn, kk, REV),
-                                                           k0 + kk, p, id, live, warp_live);
+                                                           staged_record(rec, kn, kk, REV), k0 + kk,
+                                                           p, id, live, warp_live);
+                    check = false;
                 }
             }
         }
@@ -322,19 +371,19 @@ __device__ __forceinline__ void track_chunk(const TrackChunk &c) {
     }
 }
 
-// At most two particles per thread the kernel fits 64 registers without
-// spills, i.e. 8 blocks of 128 threads per SM; four per thread need more.
+// Up to 128 registers, two blocks of 256 threads per SM: FP64 results are
+// ready after 8 cycles and one instruction keeps the pipe busy for two, so
+// two warps per scheduler nearly fill it and what counts is that ptxas has
+// the registers to load the records of the next turns ahead.  Cycles per
+// warp and turn with 1, 2, 4 and 8 warps per scheduler, one particle per
+// thread (the FP64 instructions alone: 38 / 66):
+//     exact, mu = 0      56.4  48.4  45.5  44.3   (before: 69.9  53.2  50.9  48.9)
+//     exact, mu != 0     80.7  74.8  72.7  71.6   (before: 91.9  79.9  76.4  74.6)
+// Before: per-turn looks, runs of 32 turns, 64 registers.  With 64 registers
+// the blocks of turns took 68.3, 48.8, 47.1 and 44.9 at mu = 0.
 template <int ARITH, bool OCT, bool REV, int K, bool STAGED, bool KICK>
-__global__ void __launch_bounds__(256, K <= 2 ? 4 : 1) track_chunk_kernel(const TrackChunk c) {
+__global__ void __launch_bounds__(256, K <= 2 ? 2 : 1) track_chunk_kernel(const TrackChunk c) {
     track_chunk<ARITH, OCT, REV, K, STAGED, KICK>(c);
-}
-
-// Staged fast arithmetic with two particles per thread, capped at 56
-// registers (9 blocks of 128 threads per SM): 76.5 % of the FP64 peak on
-// the DA scan against 74.5 % at 64.  Exact arithmetic gains nothing there.
-template <int ARITH, bool OCT, bool REV>
-__global__ void __maxnreg__(56) track_chunk_kernel_r56(const TrackChunk c) {
-    track_chunk<ARITH, OCT, REV, 2, true, false>(c);
 }
 
 template <int ARITH, bool OCT, bool REV, int K, bool KICK>
@@ -344,8 +393,6 @@ cudaError_t launch_s(const TrackChunk &c, unsigned blocks, int threads, cudaStre
     } else {
         const size_t smem = staged_smem_bytes(c.stage_turns, uint32_t(threads), K, KICK);
         auto kernel = track_chunk_kernel<ARITH, OCT, REV, K, true, KICK>;
-        if constexpr (ARITH == HM_ARITH_FAST && K == 2 && !KICK)
-            kernel = track_chunk_kernel_r56<ARITH, OCT, REV>;
         // Dynamic plus static shared memory above 48 KB needs the opt-in
         // (the kernel's static part is its two mbarriers): 256 threads with
         // four particles each and 256-turn stages take exactly 48 KB dynamic.
@@ -374,10 +421,12 @@ int sm_count() {
     return v;
 }
 
+constexpr uint64_t kMinBlocksPerSm = 2u;
+
 template <int ARITH, bool OCT, bool REV>
 cudaError_t launch_k(const TrackChunk &c, const TrackLaunch &l, uint32_t n_upper,
                      cudaStream_t s) {
-    const int threads = l.threads;
+    int threads = l.threads;
     if (!isnan(c.kick_module)) {
         // Kicked turns are dominated by the integer work of the generator:
         // one particle per thread.
@@ -390,10 +439,15 @@ cudaError_t launch_k(const TrackChunk &c, const TrackLaunch &l, uint32_t n_upper
     // particle is one serial chain of turns whatever its thread holds), so
     // K is halved while the grid would give fewer than two blocks per SM.
     int K = l.per_thread;
-    const uint64_t min_blocks = 2u * uint64_t(sm_count());
+    const uint64_t min_blocks = kMinBlocksPerSm * uint64_t(sm_count());
     while (K > 1 && (uint64_t(n_upper) + uint64_t(threads) * K - 1) / (uint64_t(threads) * K) <
                         min_blocks)
         K /= 2;
+    // Likewise smaller blocks: they spread a short list more evenly (40,000
+    // particles in blocks of 128 give some SMs three blocks, most two).
+    while (threads > 32 && threads % 64 == 0 &&
+           (uint64_t(n_upper) + uint64_t(threads) * K - 1) / (uint64_t(threads) * K) < min_blocks)
+        threads /= 2;
     const uint64_t per_block = uint64_t(threads) * uint64_t(K);
     const unsigned blocks = unsigned((uint64_t(n_upper) + per_block - 1) / per_block);
     if (blocks == 0) return cudaSuccess;
