@@ -3,6 +3,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <memory>
 #include <string>
 #include <vector>
 
@@ -248,26 +249,17 @@ hm_status hm_batch_create(size_t n_sets, const hm_batch_set *sets, hm_batch **ou
     auto *b = new hm_batch();
     b->params.assign(sets, sets + n_sets);
     b->offsets.assign(1, 0);
-    std::vector<double> records;
+    std::vector<hm::TableSpec> specs;
     std::vector<uint64_t> table_off;
+    uint64_t n_records = 0;  // turns of all the sets' tables
     for (size_t k = 0; k < n_sets; ++k) {
         const hm_batch_set &p = sets[k];
         b->kinds.emplace_back(p.modulation_kind ? p.modulation_kind : "sps");
-        std::vector<double> wx, wy;
-        hm_status s = hm::modulation(b->kinds.back(), p.n_turns, p.omega_x, p.omega_y, p.omega_0,
-                                     p.epsilon, p.offset, wx, wy);
-        if (s != HM_OK) {
-            delete b;
-            return s;
-        }
-        table_off.push_back(records.size());
-        for (size_t i = 0; i < wx.size(); ++i) {
-            // sin/cos of omega(n) with the host libm (src/henon.cu:2679-2682)
-            records.push_back(std::sin(wx[i]));
-            records.push_back(std::cos(wx[i]));
-            records.push_back(std::sin(wy[i]));
-            records.push_back(std::cos(wy[i]));
-        }
+        const size_t turns = hm::table_turns(b->kinds.back(), p.n_turns, p.offset);
+        specs.push_back({b->kinds.back(), uint32_t(turns), p.omega_x, p.omega_y, p.omega_0,
+                         p.epsilon, p.offset, nullptr});
+        table_off.push_back(4 * n_records);
+        n_records += turns;
         b->offsets.push_back(b->offsets.back() + p.n_particles);
         b->max_turns = std::max(b->max_turns, p.n_turns);
     }
@@ -277,7 +269,16 @@ hm_status hm_batch_create(size_t n_sets, const hm_batch_set *sets, hm_batch **ou
         return fail(HM_ERR_INVALID_ARG, "too many particles in the batch (max 2^32-1)");
     }
     b->table_off = table_off;
-    auto s = hm::upload(b->tables, records);
+    // Not a vector: its pages are first touched by the threads that fill it.
+    const std::unique_ptr<double[]> records(new double[4 * n_records]);
+    for (size_t k = 0; k < n_sets; ++k) specs[k].records = records.get() + table_off[k];
+    hm_status s = hm::turn_records(specs);
+    if (s == HM_OK) s = b->tables.alloc(4 * n_records * sizeof(double));
+    if (s == HM_OK && n_records) {
+        const cudaError_t e = cudaMemcpy(b->tables.ptr, records.get(),
+                                         4 * n_records * sizeof(double), cudaMemcpyHostToDevice);
+        if (e != cudaSuccess) s = hm::cuda_fail(e, "turn records upload");
+    }
     const size_t n = b->n_total;
     DeviceBuffer *dbl[8] = {&b->x0, &b->px0, &b->y0, &b->py0, &b->x, &b->px, &b->y, &b->py};
     for (auto *d : dbl)

@@ -175,6 +175,7 @@ DeviceBuffer &DeviceBuffer::operator=(DeviceBuffer &&o) noexcept {
         ptr = o.ptr;
         bytes = o.bytes;
         device = o.device;
+        owned = o.owned;
         o.ptr = nullptr;
         o.bytes = 0;
     }
@@ -184,7 +185,7 @@ DeviceBuffer &DeviceBuffer::operator=(DeviceBuffer &&o) noexcept {
 DeviceBuffer::~DeviceBuffer() { release(); }
 
 void DeviceBuffer::release() {
-    if (ptr) {
+    if (ptr && owned) {
         // As cudaFree: every use of the block, on any stream, ends before
         // the pool may hand it out again.
         DeviceGuard guard(device);
@@ -193,6 +194,17 @@ void DeviceBuffer::release() {
     }
     ptr = nullptr;
     bytes = 0;
+    owned = true;
+}
+
+void DeviceBuffer::part_of(const DeviceBuffer &whole, size_t nbytes, size_t *offset) {
+    release();
+    if (nbytes == 0) return;
+    ptr = static_cast<char *>(whole.ptr) + *offset;
+    bytes = nbytes;
+    device = whole.device;
+    owned = false;
+    *offset += align256(nbytes);
 }
 
 hm_status DeviceBuffer::alloc(size_t nbytes) {
@@ -512,40 +524,16 @@ using hm::ok;
 
 namespace {
 
-hm_status upload_tables(hm_tracker *t, const std::vector<double> &wx,
-                        const std::vector<double> &wy) {
-    const size_t n = wx.size();
-    t->sx.resize(n);
-    t->cx.resize(n);
-    t->sy.resize(n);
-    t->cy.resize(n);
-    // sin/cos of omega(n) with the host libm (src/henon.cu:2672-2686).
-    for (size_t i = 0; i < n; ++i) {
-        t->sx[i] = std::sin(wx[i]);
-        t->cx[i] = std::cos(wx[i]);
-        t->sy[i] = std::sin(wy[i]);
-        t->cy[i] = std::cos(wy[i]);
-    }
-    std::vector<double> rec(4 * n);
-    for (size_t i = 0; i < n; ++i) {
-        rec[4 * i + 0] = t->sx[i];
-        rec[4 * i + 1] = t->cx[i];
-        rec[4 * i + 2] = t->sy[i];
-        rec[4 * i + 3] = t->cy[i];
-    }
-    HM_TRY(t->table.alloc(rec.size() * sizeof(double)));
-    if (n) HM_CUDA_TRY(cudaMemcpy(t->table.ptr, rec.data(), rec.size() * sizeof(double),
-                                  cudaMemcpyHostToDevice));
-    t->allowed_steps = n;
-    return ok();
-}
-
 hm_status compute_tables(hm_tracker *t, uint32_t n_turns, double omega_x, double omega_y,
                          const char *kind, double omega_0, double epsilon, uint32_t offset) {
     if (!kind) return fail(HM_ERR_INVALID_ARG, "null modulation kind");
-    std::vector<double> wx, wy;
-    HM_TRY(hm::modulation(kind, n_turns, omega_x, omega_y, omega_0, epsilon, offset, wx, wy));
-    HM_TRY(upload_tables(t, wx, wy));
+    const size_t n = hm::table_turns(kind, n_turns, offset);
+    std::vector<double> records(4 * n);
+    HM_TRY(hm::turn_records({{kind, uint32_t(n), omega_x, omega_y, omega_0, epsilon, offset,
+                              records.data()}}));
+    t->records = std::move(records);
+    HM_TRY(hm::upload(t->table, t->records));
+    t->allowed_steps = n;
     {
         // the adjoint's ripple follows the modulation
         std::lock_guard<std::mutex> lock(t->adjoint_mutex);
@@ -572,15 +560,21 @@ hm_status particles_upload(hm_particles *p, const double *x, const double *px,
     hm::DeviceBuffer *cur[4] = {&p->x, &p->px, &p->y, &p->py};
     hm::DeviceBuffer *ini[4] = {&p->x0d, &p->px0d, &p->y0d, &p->py0d};
     const double *src[4] = {x, px, y, py};
+    // One block for the thirteen arrays: an allocation waits for its stream
+    // and a release for the device, 6-8 us each (150 us a set before).
+    using hm::align256;
+    HM_TRY(p->slab.alloc(8 * align256(n * sizeof(double)) + align256(n * sizeof(uint32_t)) +
+                         2 * align256(n) + 2 * align256(n * sizeof(uint64_t))));
+    size_t at = 0;
     for (int f = 0; f < 4; ++f) {
-        HM_TRY(cur[f]->alloc(n * sizeof(double)));
-        HM_TRY(ini[f]->alloc(n * sizeof(double)));
+        cur[f]->part_of(p->slab, n * sizeof(double), &at);
+        ini[f]->part_of(p->slab, n * sizeof(double), &at);
     }
-    HM_TRY(p->steps.alloc(n * sizeof(uint32_t)));
-    HM_TRY(p->dvalid.alloc(n));
-    HM_TRY(p->dghost.alloc(n));
-    HM_TRY(p->didx.alloc(n * sizeof(uint64_t)));
-    HM_TRY(p->didx_base.alloc(n * sizeof(uint64_t)));
+    p->steps.part_of(p->slab, n * sizeof(uint32_t), &at);
+    p->dvalid.part_of(p->slab, n, &at);
+    p->dghost.part_of(p->slab, n, &at);
+    p->didx.part_of(p->slab, n * sizeof(uint64_t), &at);
+    p->didx_base.part_of(p->slab, n * sizeof(uint64_t), &at);
     if (n == 0) return ok();
     const cudaStream_t s = 0;
     for (int f = 0; f < 4; ++f) {
@@ -772,12 +766,15 @@ hm_status hm_tracker_allowed_steps(const hm_tracker *t, uint64_t *out) {
 hm_status hm_tracker_get_tables(const hm_tracker *t, double *sin_x, double *cos_x, double *sin_y,
                                 double *cos_y) {
     if (!t) return fail(HM_ERR_INVALID_ARG, "null tracker");
-    const size_t n = t->sx.size();
+    const size_t n = t->records.size() / 4;
     if (n && (!sin_x || !cos_x || !sin_y || !cos_y)) return fail(HM_ERR_INVALID_ARG, "null pointer");
-    std::memcpy(sin_x, t->sx.data(), n * sizeof(double));
-    std::memcpy(cos_x, t->cx.data(), n * sizeof(double));
-    std::memcpy(sin_y, t->sy.data(), n * sizeof(double));
-    std::memcpy(cos_y, t->cy.data(), n * sizeof(double));
+    for (size_t i = 0; i < n; ++i) {
+        const double *const r = t->records.data() + 4 * i;
+        sin_x[i] = r[0];
+        cos_x[i] = r[1];
+        sin_y[i] = r[2];
+        cos_y[i] = r[3];
+    }
     return ok();
 }
 

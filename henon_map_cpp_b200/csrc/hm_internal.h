@@ -46,6 +46,19 @@ hm_status modulation(const std::string &kind, uint32_t n_turns, double omega_x,
                      double omega_y, double omega_0, double epsilon,
                      uint32_t offset, std::vector<double> &wx,
                      std::vector<double> &wy);
+// Turns of a table: the span offset .. offset + n_turns as the reference's
+// 32-bit integers see it, for the kinds that are functions of the turn.
+size_t table_turns(const std::string &kind, uint32_t n_turns, uint32_t offset);
+// One table of turn records {sin wx, cos wx, sin wy, cos wy}, n_turns (from
+// table_turns) of them written to `records`.
+struct TableSpec {
+    std::string kind;
+    uint32_t n_turns;
+    double omega_x, omega_y, omega_0, epsilon;
+    uint32_t offset;
+    double *records;
+};
+hm_status turn_records(const std::vector<TableSpec> &specs);
 std::vector<double> birkhoff_weights(uint32_t n);
 hm_status modulation_ripple(const std::string &kind, uint32_t n_turns, double omega_0,
                             uint32_t offset, std::vector<double> &ripple);
@@ -61,10 +74,12 @@ struct DeviceBuffer {
     void *ptr = nullptr;
     size_t bytes = 0;
     int device = 0;
+    bool owned = true;
     DeviceBuffer() = default;
     DeviceBuffer(const DeviceBuffer &) = delete;
     DeviceBuffer &operator=(const DeviceBuffer &) = delete;
-    DeviceBuffer(DeviceBuffer &&o) noexcept : ptr(o.ptr), bytes(o.bytes), device(o.device) {
+    DeviceBuffer(DeviceBuffer &&o) noexcept
+        : ptr(o.ptr), bytes(o.bytes), device(o.device), owned(o.owned) {
         o.ptr = nullptr;
         o.bytes = 0;
     }
@@ -72,6 +87,9 @@ struct DeviceBuffer {
     ~DeviceBuffer();
     hm_status alloc(size_t nbytes);    // frees any previous allocation
     hm_status ensure(size_t nbytes);   // grows (never shrinks)
+    // Becomes nbytes of `whole` at *offset, which moves to the next multiple
+    // of 256; `whole` stays the owner and has to live longer.
+    void part_of(const DeviceBuffer &whole, size_t nbytes, size_t *offset);
     void release();
     template <class T> T *as() const { return static_cast<T *>(ptr); }
 };
@@ -96,6 +114,7 @@ struct hm_particles {
     uint32_t live_step = 0;
     // Device state, and the initial conditions on the device (reset
     // restarts from them).  The device copies are authoritative.
+    hm::DeviceBuffer slab;  // one allocation for all of them
     hm::DeviceBuffer x, px, y, py, steps, dvalid, dghost, didx, didx_base;
     hm::DeviceBuffer x0d, px0d, y0d, py0d;
     // Host mirrors of what the reference keeps on the host side (initial
@@ -117,8 +136,8 @@ struct hm_particles {
 // Modulation tables on the device (henon_tracker_gpu, src/henon.h:212-228).
 struct hm_tracker {
     uint64_t allowed_steps = 0;
-    std::vector<double> sx, cx, sy, cy;  // host copies
-    hm::DeviceBuffer table;              // {sx, cx, sy, cy} per turn
+    std::vector<double> records;  // {sx, cx, sy, cy} per turn, host copy
+    hm::DeviceBuffer table;       // the same on the device
     hm_arith arith = HM_ARITH_EXACT;
     // Modulation parameters the tables were built from (for derivatives).
     std::string kind = "sps";
@@ -139,7 +158,7 @@ namespace hm {
 
 // High word of the largest coordinate bound t for which a state with all
 // |coordinates| < t cannot be one turn past a state outside the barrier
-// (dev::run_turns): g(2t) = R + R^2 + |mu| R^3 < barrier at R = 2t.  R is
+// (dev::block_turns): g(2t) = R + R^2 + |mu| R^3 < barrier at R = 2t.  R is
 // found from above by Newton's method (g is convex and increasing, so the
 // iterates stay above the root) and then shrunk until g(R) is below the
 // barrier less 2^-8 of it.  That margin covers the roundings of a turn (a

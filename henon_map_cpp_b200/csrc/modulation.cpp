@@ -5,7 +5,10 @@
 // (src/modulation.cpp:3-134, src/henon.cu:2657-2694): the device only reads
 // the resulting tables, so the expression order below is chosen to give
 // bit-identical doubles to the reference on the same host.
+#include <algorithm>
+#include <atomic>
 #include <cmath>
+#include <exception>
 #include <random>
 #include <string>
 #include <thread>
@@ -24,22 +27,44 @@ constexpr double kSpsCoefficient[kSpsHarmonics] = {
     1.000e-4, 0.218e-4, 0.708e-4, 0.254e-4, 0.100e-4, 0.078e-4, 0.218e-4};
 constexpr int kSpsMultiple[kSpsHarmonics] = {1, 2, 3, 6, 7, 10, 12};
 
-// Runs body(i) for i in [0, n) on all host threads, interleaved.
-template <class F> void parallel_for(size_t n, F body) {
-    unsigned n_threads = std::thread::hardware_concurrency();
-    if (n_threads == 0) n_threads = 1;
-    if (n < 4096 || n_threads == 1) {
-        for (size_t i = 0; i < n; ++i) body(i);
-        return;
-    }
+// Runs body(lo, hi) over [0, n) in pieces of kPiece, dealt to the host's
+// threads (this one among them) by a counter.  A thread that cannot be
+// started is done without.  Starting one costs 20-30 us, as much as about a
+// thousand turns' sines and cosines, so small ranges take few.
+constexpr size_t kPiece = 1024;
+
+template <class F> void parallel_pieces(size_t n, F body) {
+    const size_t pieces = (n + kPiece - 1) / kPiece;
+    const size_t hw = std::max<size_t>(1, std::thread::hardware_concurrency());
+    std::atomic<size_t> next{0};
+    auto work = [&] {
+        for (size_t q; (q = next.fetch_add(1)) < pieces;)
+            body(q * kPiece, std::min(n, (q + 1) * kPiece));
+    };
     std::vector<std::thread> pool;
-    pool.reserve(n_threads);
-    for (unsigned t = 0; t < n_threads; ++t)
-        pool.emplace_back([=, &body] {
-            for (size_t i = t; i < n; i += n_threads) body(i);
-        });
+    try {
+        while (pool.size() + 1 < std::min(hw, pieces)) pool.emplace_back(work);
+    } catch (const std::exception &) {
+    }
+    work();
     for (auto &th : pool) th.join();
 }
+
+// The SPS ripple sum_j c_j cos(Omega_j * turn), harmonics summed in
+// ascending j (sps_modulation, src/modulation.cpp:31-60).
+struct SpsRipple {
+    double omega_k[kSpsHarmonics];
+    SpsRipple() {
+        const double fundamental = 2 * M_PI / 868.12;
+        for (int j = 0; j < kSpsHarmonics; ++j) omega_k[j] = double(kSpsMultiple[j]) * fundamental;
+    }
+    double operator()(double turn) const {
+        double ripple = 0.0;
+        for (int j = 0; j < kSpsHarmonics; ++j)
+            ripple += kSpsCoefficient[j] * std::cos(omega_k[j] * turn);
+        return ripple;
+    }
+};
 
 }  // namespace
 
@@ -49,19 +74,14 @@ template <class F> void parallel_for(size_t n, F body) {
 std::vector<double> sps_modulation(double tune, double epsilon, int32_t start,
                                    int32_t end) {
     std::vector<double> out(end > start ? size_t(end - start) : 0);
-    double omega_k[kSpsHarmonics];
-    const double fundamental = 2 * M_PI / 868.12;
-    for (int j = 0; j < kSpsHarmonics; ++j)
-        omega_k[j] = double(kSpsMultiple[j]) * fundamental;
+    const SpsRipple ripple;
     const double two_pi_tune = 2 * M_PI * tune;
-    parallel_for(out.size(), [&](size_t i) {
+    parallel_pieces(out.size(), [&](size_t lo, size_t hi) {
         // The reference adds an unsigned index to the int start: the turn
         // number is formed in 32-bit unsigned arithmetic.
-        const double turn = double(uint32_t(uint32_t(i) + uint32_t(start)));
-        double ripple = 0.0;
-        for (int j = 0; j < kSpsHarmonics; ++j)
-            ripple += kSpsCoefficient[j] * std::cos(omega_k[j] * turn);
-        out[i] = two_pi_tune * (1 + epsilon * ripple);
+        for (size_t i = lo; i < hi; ++i)
+            out[i] = two_pi_tune *
+                     (1 + epsilon * ripple(double(uint32_t(uint32_t(i) + uint32_t(start)))));
     });
     return out;
 }
@@ -121,6 +141,52 @@ hm_status modulation(const std::string &kind, uint32_t n_turns, double omega_x,
     return ok();
 }
 
+size_t table_turns(const std::string &kind, uint32_t n_turns, uint32_t offset) {
+    if (kind != "sps" && kind != "basic") return n_turns;
+    const int32_t start = int32_t(offset), end = int32_t(offset + n_turns);
+    return end > start ? size_t(end - start) : 0;
+}
+
+// sin and cos of omega(n) with the host libm (src/henon.cu:2672-2686), for
+// several tables at once on all host threads.  SPS angles are formed where
+// their sines are taken, both planes from one ripple sum; the other kinds
+// (two of them draw random tunes in order) are formed first.
+hm_status turn_records(const std::vector<TableSpec> &specs) {
+    std::vector<std::vector<double>> wx(specs.size()), wy(specs.size());
+    std::vector<size_t> first(1, 0);
+    for (size_t k = 0; k < specs.size(); ++k) {
+        const TableSpec &t = specs[k];
+        if (t.kind != "sps")
+            HM_TRY(modulation(t.kind, t.n_turns, t.omega_x, t.omega_y, t.omega_0, t.epsilon,
+                              t.offset, wx[k], wy[k]));
+        first.push_back(first.back() + t.n_turns);
+    }
+    const SpsRipple ripple;
+    parallel_pieces(first.back(), [&](size_t lo, size_t hi) {
+        size_t k = size_t(std::upper_bound(first.begin(), first.end(), lo) - first.begin()) - 1;
+        for (size_t g = lo; g < hi; ++g) {
+            while (g >= first[k + 1]) ++k;
+            const TableSpec &t = specs[k];
+            const size_t i = g - first[k];
+            double ox, oy;
+            if (wx[k].empty()) {
+                const double r = 1 + t.epsilon * ripple(double(uint32_t(uint32_t(i) + t.offset)));
+                ox = 2 * M_PI * t.omega_x * r;
+                oy = 2 * M_PI * t.omega_y * r;
+            } else {
+                ox = wx[k][i];
+                oy = wy[k][i];
+            }
+            double *const rec = t.records + 4 * i;
+            rec[0] = std::sin(ox);
+            rec[1] = std::cos(ox);
+            rec[2] = std::sin(oy);
+            rec[3] = std::cos(oy);
+        }
+    });
+    return ok();
+}
+
 // The ripple S_n of omega(n) = 2*pi*tune*(1 + eps*S_n) for the kinds whose
 // angle is differentiable in (tune, eps): "sps" (the harmonic sum above) and
 // "basic" (cos(2*pi*omega_0*i)).
@@ -128,15 +194,9 @@ hm_status modulation_ripple(const std::string &kind, uint32_t n_turns, double om
                             uint32_t offset, std::vector<double> &ripple) {
     ripple.assign(n_turns, 0.0);
     if (kind == "sps") {
-        double omega_k[kSpsHarmonics];
-        const double fundamental = 2 * M_PI / 868.12;
-        for (int j = 0; j < kSpsHarmonics; ++j)
-            omega_k[j] = double(kSpsMultiple[j]) * fundamental;
-        parallel_for(n_turns, [&](size_t i) {
-            const double turn = double(uint32_t(uint32_t(i) + offset));
-            double s = 0.0;
-            for (int j = 0; j < kSpsHarmonics; ++j) s += kSpsCoefficient[j] * std::cos(omega_k[j] * turn);
-            ripple[i] = s;
+        const SpsRipple sps;
+        parallel_pieces(n_turns, [&](size_t lo, size_t hi) {
+            for (size_t i = lo; i < hi; ++i) ripple[i] = sps(double(uint32_t(uint32_t(i) + offset)));
         });
         return ok();
     }

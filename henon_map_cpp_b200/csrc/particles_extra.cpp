@@ -266,15 +266,15 @@ hm_status hm_tracker_tangent_matrices(const hm_tracker *t, const hm_particles *p
     HM_CUDA_TRY(cudaMemcpy(px.data(), p->px.ptr, n * sizeof(double), cudaMemcpyDeviceToHost));
     HM_CUDA_TRY(cudaMemcpy(y.data(), p->y.ptr, n * sizeof(double), cudaMemcpyDeviceToHost));
     HM_CUDA_TRY(cudaMemcpy(py.data(), p->py.ptr, n * sizeof(double), cudaMemcpyDeviceToHost));
+    const double *const rec = t->records.data() + 4 * size_t(s);
     for (size_t i = 0; i < n; ++i) {
         double *m = host_out + 16 * i;
         if (!p->valid[i]) {
             for (int k = 0; k < 16; ++k) m[k] = std::nan("");
         } else if (!reverse) {
-            tangent_host(x[i], y[i], t->sx[s], t->cx[s], t->sy[s], t->cy[s], mu, m);
+            tangent_host(x[i], y[i], rec[0], rec[1], rec[2], rec[3], mu, m);
         } else {
-            inverse_tangent_host(x[i], px[i], y[i], py[i], t->sx[s], t->cx[s], t->sy[s],
-                                 t->cy[s], mu, m);
+            inverse_tangent_host(x[i], px[i], y[i], py[i], rec[0], rec[1], rec[2], rec[3], mu, m);
         }
     }
     return ok();
