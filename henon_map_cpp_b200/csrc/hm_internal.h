@@ -426,8 +426,12 @@ struct OrbitRecordArgs {
     uint32_t live_step, n_turns;
     double mu;
     long long b2bits;
+    uint32_t pair_hi;  // pair_threshold_hi(barrier^2, mu)
     int arith;
-    double *ox, *opx, *oy, *opy;  // orbit [n][n_turns + 1] (each particle's samples contiguous)
+    // Orbit: each particle's n_turns + 1 samples contiguous, `pitch` doubles
+    // from one particle's to the next's.
+    double *ox, *opx, *oy, *opy;
+    size_t pitch;
     // Optional (null when unused): each coordinate's sum over the samples,
     // from 0.0 in sample order ([4][n]), and the first sample holding NaN
     // (n_turns + 1 when none).
@@ -449,7 +453,8 @@ cudaError_t launch_orbit_record(const OrbitRecordArgs &a, cudaStream_t s);
 // segments in order.  Coordinates have means[c * n + i] subtracted first
 // when means is not null.
 struct BirkhoffSegArgs {
-    const double *x, *px, *y, *py;  // orbit [n][S]
+    const double *x, *px, *y, *py;  // orbit [n][pitch], S samples each
+    size_t pitch;
     const double *means;            // [4][n] or null
     const uint32_t *first_nan;      // [n]
     size_t n, S;
@@ -473,7 +478,7 @@ cudaError_t launch_hann_table(double *h, uint32_t len, cudaStream_t s);
 cudaError_t launch_fft_gather2(const double *x, const double *px, const double *y,
                                const double *py, const double *means, size_t n, uint32_t from,
                                uint32_t len, const double *h, double2 *z, size_t S,
-                               cudaStream_t s);
+                               size_t pitch, cudaStream_t s);
 cudaError_t launch_fft_peak2(const double2 *z, uint32_t len, size_t n, uint32_t last_sample,
                              const uint32_t *first_nan, double *out, size_t cols, int col,
                              cudaStream_t s);

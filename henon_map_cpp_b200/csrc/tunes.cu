@@ -40,31 +40,79 @@ using dev::Rn;
 // turn is the tracker's: forward with table[live_step + k], or backward with
 // table[live_step - 1 - k] (REV), with the tracker's reproducible kicks
 // (KICK: added before the forward turn, subtracted after the backward
-// one).  Optionally each coordinate's sum over the samples (from 0.0, in
-// sample order: the reference's std::accumulate for all_tunes' mean,
+// one).  Also each coordinate's sum over the samples (from 0.0, in sample
+// order: the reference's std::accumulate for all_tunes' mean,
 // src/henon.cu:3040-3051) and the first NaN sample.
-// The orbit is particle-major, so a warp's samples of one turn would land
-// in 32 different rows: each lane collects kRecGroup samples in shared
-// memory and the warp then writes them out as whole 128-byte lines (lanes
-// 0-15 one particle's run, lanes 16-31 the next).  Lanes past the last
-// particle run the loop on zeros (a fixed point) and write nothing.
-constexpr uint32_t kRecGroup = 16;
-
-__host__ __device__ constexpr size_t record_smem_bytes(int threads) {
-    return size_t(threads) * 4u * (kRecGroup + 1u) * sizeof(double);  // +1: bank padding
-}
+//
+// A tune call has few particles (16,384 are 3.5 warps per SM) and each orbit
+// is one serial chain of turns, so the time is that of one warp's turns.
+// Two warps share the work of 32 particles: the first runs the turns in
+// groups of 16 samples without per-turn control flow (dev::block_turns'
+// scheme, with a redo of the group where a coordinate was large) and puts
+// each sample into shared memory; the second writes the group before to the
+// orbit as whole 128-byte lines (the orbit is particle-major, so a warp's
+// samples of one turn would land in 32 different rows) and brings in the
+// turn records of the group after next.  One block barrier per group.
+// 16,384 particles x 1e4 turns: 3.39 ms with one warp doing all of it and
+// testing every turn (528 cycles a turn), 1.32 ms now, bound by the 5.2 GB
+// that it writes (0.62 ms with 2,048 particles).
+// Lanes past the last particle run the loop on zeros (a fixed point) and
+// write nothing.
+constexpr uint32_t kRecGroup = dev::kBlockTurns;
+constexpr uint32_t kRecRow = kRecGroup + 1u;  // a lane's samples, padded for the banks
+constexpr uint32_t kRecBuf = 4u * 32u * kRecRow;  // doubles of a group: [coordinate][lane][sample]
 
 template <int ARITH, bool OCT, bool REV, bool KICK>
-__global__ void orbit_record_kernel(OrbitRecordArgs a) {
-    extern __shared__ double rec_stage[];  // [warp][coordinate][lane (kRecGroup + 1)]
-    const size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    const bool valid = i < a.n;
-    const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+__global__ void __launch_bounds__(64) orbit_record_kernel(OrbitRecordArgs a) {
+    __shared__ __align__(16) double samples[2][kRecBuf];
+    __shared__ __align__(16) double2 recs[2][2u * kRecGroup];
+    const unsigned lane = threadIdx.x & 31u;
+    const size_t first = size_t(blockIdx.x) * 32u, i = first + lane;
     const size_t n = a.n, S = size_t(a.n_turns) + 1u;
-    const size_t first_of_warp = i - lane;
-    constexpr uint32_t G = kRecGroup, W = G + 1u;
-    double *st = rec_stage + size_t(warp) * 4u * 32u * W;
-    double x = 0.0, px = 0.0, y = 0.0, py = 0.0;
+    const bool valid = i < n;
+    const uint32_t groups = uint32_t((S + kRecGroup - 1u) / kRecGroup);
+    constexpr uint32_t G = kRecGroup, W = kRecRow;
+
+    if (threadIdx.x >= 32u) {
+        // ---- the writing warp ------------------------------------------------
+        // Lane l brings in half l & 1 of the record of the group's turn l / 2
+        // (zeros past the last turn, which no turn reads).
+        auto fetch = [&](uint32_t g) {
+            const uint32_t k = g * G + (lane >> 1);
+            if (k >= a.n_turns) return make_double2(0.0, 0.0);
+            const uint32_t idx = REV ? a.live_step - 1u - k : a.live_step + k;
+            return __ldg(reinterpret_cast<const double2 *>(a.table) + 2u * size_t(idx) +
+                         (lane & 1u));
+        };
+        recs[0][lane] = fetch(0u);
+        recs[1][lane] = fetch(1u);
+        __syncthreads();
+        double2 next = fetch(2u);
+        for (uint32_t g = 0; g < groups; ++g) {
+            __syncthreads();  // group g is complete, its records are used
+            recs[g & 1u][lane] = next;
+            next = fetch(g + 3u);
+            const double *st = samples[g & 1u];
+            const uint32_t base = g * G, cnt = uint32_t(S - base < G ? S - base : G);
+            // lanes 0-15 one particle's samples, lanes 16-31 the next one's
+            const uint32_t gg = lane % G;
+            size_t o = (first + lane / G) * a.pitch + base + gg;
+            const double *src = st + (lane / G) * W + gg;
+            if (gg < cnt)
+#pragma unroll 4
+                for (uint32_t pl = lane / G; pl < 32u && first + pl < n;
+                     pl += 32u / G, o += (32u / G) * a.pitch, src += (32u / G) * W) {
+                    a.ox[o] = src[0];
+                    a.opx[o] = src[32u * W];
+                    a.oy[o] = src[2u * 32u * W];
+                    a.opy[o] = src[3u * 32u * W];
+                }
+        }
+        return;
+    }
+
+    // ---- the tracking warp ---------------------------------------------------
+    double x = 0.0, px = 0.0, y = 0.0, py = 0.0;  // what a lost lane records
     uint32_t steps = 0;
     if (valid) {
         x = a.x[i];
@@ -76,85 +124,101 @@ __global__ void orbit_record_kernel(OrbitRecordArgs a) {
     bool alive = valid && !dev::is_lost(x, px, y, py);
     uint32_t first_nan = alive ? a.n_turns + 1u : 0u;
     double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
-    const bool sums = a.sums != nullptr;
-    // Sample s of this lane into the stage; the warp writes a full group
-    // (or the last, partial one) out.
-    auto put = [&](uint32_t s) {
-        const uint32_t g = s % G;
-        st[0 * 32u * W + lane * W + g] = x;
-        st[1 * 32u * W + lane * W + g] = px;
-        st[2 * 32u * W + lane * W + g] = y;
-        st[3 * 32u * W + lane * W + g] = py;
-        if (sums) {
-            s0 = Rn::add(s0, x);
-            s1 = Rn::add(s1, px);
-            s2 = Rn::add(s2, y);
-            s3 = Rn::add(s3, py);
-        }
-        if (g == G - 1u || s == a.n_turns) {
-            __syncwarp();
-            const uint32_t base = s - g, cnt = g + 1u;
+    dev::Particle p[1] = {alive ? dev::make_particle(x, px, y, py)
+                                : dev::make_particle(0.0, 0.0, 0.0, 0.0)};
+    const dev::Barrier bar = dev::make_barrier<ARITH>(a.b2bits);
+    const double mu = a.mu;
+    __syncthreads();
+    for (uint32_t g = 0; g < groups; ++g) {
+        const uint32_t k0 = g * G;
+        const uint32_t cnt = uint32_t(S - k0 < G ? S - k0 : G);  // samples of the group
+        double *const st = samples[g & 1u] + lane * W;
+        const double2 *const q = recs[g & 1u];
+        auto put = [&](uint32_t u, double v0, double v1, double v2, double v3) {
+            st[u] = v0;
+            st[32u * W + u] = v1;
+            st[2u * 32u * W + u] = v2;
+            st[3u * 32u * W + u] = v3;
+            s0 = Rn::add(s0, v0);
+            s1 = Rn::add(s1, v1);
+            s2 = Rn::add(s2, v2);
+            s3 = Rn::add(s3, v3);
+        };
+        const dev::Particle from = p[0];
+        const double f0 = s0, f1 = s1, f2 = s2, f3 = s3;
+        // Each sample is the state before its turn.
+        const bool whole = !KICK && k0 + G <= a.n_turns && a.pair_hi != 0u;
+        bool redo = !whole;
+        if (whole) {
+            float big = 0.0f;
 #pragma unroll
-            for (uint32_t v = lane; v < 32u * G; v += 32u) {
-                const uint32_t pl = v / G, gg = v % G;
-                const size_t ip = first_of_warp + pl;
-                if (gg < cnt && ip < n) {
-                    const size_t o = ip * S + base + gg;
-                    a.ox[o] = st[0 * 32u * W + pl * W + gg];
-                    a.opx[o] = st[1 * 32u * W + pl * W + gg];
-                    a.oy[o] = st[2 * 32u * W + pl * W + gg];
-                    a.opy[o] = st[3 * 32u * W + pl * W + gg];
+            for (uint32_t u = 0; u < G; ++u) {
+                put(u, p[0].x, p[0].px, p[0].y, p[0].py);
+                const double2 r = q[2u * u], t = q[2u * u + 1u];
+                dev::turn<ARITH, OCT, REV>(p[0], dev::Turn{r.x, r.y, t.x, t.y}, mu);
+                if (u & 1u)
+                    big = dev::hi_max(dev::hi_max(big, p[0].x, p[0].px), p[0].y, p[0].py);
+            }
+            redo = __any_sync(dev::kFullMask,
+                              (__float_as_uint(big) & 0x7fffffffu) >= a.pair_hi);
+            // A lane lost before this group ran it on zeros; what it records
+            // stays as it was.
+            if (!redo && !alive) {
+                s0 = f0;
+                s1 = f1;
+                s2 = f2;
+                s3 = f3;
+                for (uint32_t u = 0; u < G; ++u) put(u, x, px, y, py);
+            }
+            if (!redo && alive) steps = REV ? steps - G : steps + G;
+        }
+        if (redo) {  // the group turn by turn
+            p[0] = from;
+            s0 = f0;
+            s1 = f1;
+            s2 = f2;
+            s3 = f3;
+            for (uint32_t u = 0; u < cnt; ++u) {
+                if (alive) put(u, p[0].x, p[0].px, p[0].y, p[0].py);
+                else put(u, x, px, y, py);
+                const uint32_t k = k0 + u;
+                if (k >= a.n_turns || !alive) continue;
+                const double2 r = q[2u * u], t = q[2u * u + 1u];
+                const uint32_t idx = REV ? a.live_step - 1u - k : a.live_step + k;
+                if (KICK && !REV)
+                    dev::apply_kick<false>(p[0], dev::kick_direction(a.kick_seed, a.id0 + i, idx),
+                                           a.kick_module);
+                dev::turn<ARITH, OCT, REV>(p[0], dev::Turn{r.x, r.y, t.x, t.y}, mu);
+                if (KICK && REV)
+                    dev::apply_kick<true>(p[0], dev::kick_direction(a.kick_seed, a.id0 + i, idx),
+                                          a.kick_module);
+                if (dev::inside_after_turn<ARITH>(p[0], bar)) {
+                    steps = REV ? steps - 1u : steps + 1u;
+                } else {
+                    x = px = y = py = dev::quiet_nan();
+                    alive = false;
+                    first_nan = k + 1u;
+                    p[0] = dev::make_particle(0.0, 0.0, 0.0, 0.0);
                 }
             }
-            __syncwarp();
         }
-    };
-    put(0);
-    dev::Particle p = dev::make_particle(x, px, y, py);
-    const dev::Barrier bar = dev::make_barrier<ARITH>(a.b2bits);
-    const unsigned long long id = a.id0 + i;
-    // The next turn's record is loaded a turn ahead, off the orbit's chain.
-    auto table_index = [&](uint32_t k) { return REV ? a.live_step - 1u - k : a.live_step + k; };
-    dev::Turn t_next = a.n_turns ? dev::load_turn(a.table, table_index(0)) : dev::Turn{};
-    for (uint32_t k = 0; k < a.n_turns; ++k) {
-        const dev::Turn t = t_next;
-        if (k + 1 < a.n_turns) t_next = dev::load_turn(a.table, table_index(k + 1));
-        if (alive) {
-            const uint32_t idx = table_index(k);
-            if (KICK && !REV)
-                dev::apply_kick<false>(p, dev::kick_direction(a.kick_seed, id, idx), a.kick_module);
-            dev::turn<ARITH, OCT, REV>(p, t, a.mu);
-            if (KICK && REV)
-                dev::apply_kick<true>(p, dev::kick_direction(a.kick_seed, id, idx), a.kick_module);
-            if (dev::inside_after_turn<ARITH>(p, bar)) {
-                steps = REV ? steps - 1u : steps + 1u;
-                x = p.x;
-                px = p.px;
-                y = p.y;
-                py = p.py;
-            } else {
-                x = px = y = py = dev::quiet_nan();
-                alive = false;
-                first_nan = k + 1u;
-            }
-        }
-        put(k + 1u);
+        __syncthreads();
     }
     if (!valid) return;
-    a.x[i] = x;
-    a.px[i] = px;
-    a.y[i] = y;
-    a.py[i] = py;
+    a.x[i] = alive ? p[0].x : x;
+    a.px[i] = alive ? p[0].px : px;
+    a.y[i] = alive ? p[0].y : y;
+    a.py[i] = alive ? p[0].py : py;
     a.steps[i] = steps;
-    if (sums) {
+    if (a.sums) {
         a.sums[i] = s0;
         a.sums[n + i] = s1;
         a.sums[2 * n + i] = s2;
         a.sums[3 * n + i] = s3;
+        // With the mean removed, one NaN sample makes the mean, and so every
+        // sample, NaN.
+        if (first_nan <= a.n_turns) first_nan = 0u;
     }
-    // With the mean removed, one NaN sample makes the mean, and so every
-    // sample, NaN.
-    if (sums && first_nan <= a.n_turns) first_nan = 0u;
     if (a.first_nan) a.first_nan[i] = first_nan;
 }
 
@@ -172,15 +236,46 @@ __device__ __forceinline__ double centred(double v, const double *means, double 
     return means ? Rn::sub(v, m) : v;
 }
 
-// Birkhoff phase-advance sums of one segment of turns [s0, s1) for one plane
-// of one particle, every window at once: the transition s -> s+1 adds
-// w_j[s - from_j] dtheta_s to window j when from_j <= s < to_j, dtheta
-// wrapped by +2 pi when negative (birkhoff_tune,
-// src/dynamic_indicator.cpp:81-131).  Windows in groups of kWinGroup
-// (blockIdx.y) so that the sums stay in registers.
+// Four consecutive samples as one 32-byte load (sm_100; p 32-byte aligned).
+__device__ __forceinline__ void load4(const double *p, double (&v)[4]) {
+    asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
+        : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(v[3])
+        : "l"(p));
+}
+
+// Birkhoff phase-advance sums of one segment for one plane of one particle,
+// every window at once: the transition s -> s+1 adds w_j[s - from_j] dtheta_s
+// to window j when from_j <= s < to_j, dtheta wrapped by +2 pi when negative
+// (birkhoff_tune, src/dynamic_indicator.cpp:81-131).  A segment holds the
+// transitions into its samples [g seg_len, (g + 1) seg_len), seg_len a
+// multiple of 4.  Windows in groups of kWinGroup (blockIdx.y) so that the
+// sums stay in registers.
+//
+// Samples are taken four at a time: neighbouring threads read rows of
+// `pitch` doubles, so an 8-byte load of a warp costs 32 tag look-ups for 256
+// bytes, and this way a quarter of them.  A window that holds all four
+// transitions, or none, is told by one test instead of four.  16,384
+// particles x 1e4 turns, 4 windows and the full orbit: 2.74 ms, bound by the
+// instructions of atan2 (sample by sample, each window tested each time:
+// 4.47 ms; 3.85 once the rows were aligned).
 constexpr int kWinGroup = 8;
 
-__global__ void birkhoff_seg_kernel(const BirkhoffSegArgs a) {
+__global__ void __launch_bounds__(128, 5) birkhoff_seg_kernel(const BirkhoffSegArgs a) {
+    // The block's windows: the samples that the first and last of its
+    // transitions lead to, and the weight of a transition into sample s, w[s].
+    struct Window {
+        uint32_t first, last;
+        const double *w;
+    };
+    __shared__ Window win[kWinGroup];
+    const int w0 = int(blockIdx.y) * kWinGroup;
+    const int nw = min(kWinGroup, a.n_win - w0);
+    if (int(threadIdx.x) < nw) {
+        const uint32_t from = a.from[w0 + threadIdx.x];
+        win[threadIdx.x] = Window{from + 1u, a.to[w0 + threadIdx.x],
+                                  a.w + ((long long)a.w_off[w0 + threadIdx.x] - (long long)from - 1)};
+    }
+    __syncthreads();
     const size_t t = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
     const size_t n = a.n;
     const size_t sp = t / n;  // segment * 2 + plane
@@ -188,39 +283,43 @@ __global__ void birkhoff_seg_kernel(const BirkhoffSegArgs a) {
     const size_t i = t - sp * n;
     const uint32_t seg = uint32_t(sp >> 1);
     const int plane = int(sp & 1u);
-    const int w0 = int(blockIdx.y) * kWinGroup;
-    const int nw = min(kWinGroup, a.n_win - w0);
-    const double *q = plane ? a.y : a.x, *p = plane ? a.py : a.px;
     const double mq = mean_of(a.means, n, i, 2 * plane, a.S);
     const double mp = mean_of(a.means, n, i, 2 * plane + 1, a.S);
-    const uint32_t s0 = seg * a.seg_len;
-    const uint32_t s1 = min(uint32_t(a.S - 1), s0 + a.seg_len);
-    uint32_t lo[kWinGroup], hi[kWinGroup];
-    long long wb[kWinGroup];  // weight of transition s: w[wb + s]
-    double acc[kWinGroup];
+    double acc[kWinGroup] = {};
+    const double *const q = (plane ? a.y : a.x) + i * a.pitch;  // this particle's samples
+    const double *const p = (plane ? a.py : a.px) + i * a.pitch;
+    const uint32_t b0 = seg * a.seg_len;
+    const uint32_t b1 = uint32_t(a.S - b0 < a.seg_len ? a.S : size_t(b0) + a.seg_len);
+    double prev = 0.0;
+    if (b0 > 0u) prev = atan2(centred(p[b0 - 1u], a.means, mp), centred(q[b0 - 1u], a.means, mq));
+    // The row's padding is readable past sample S - 1; no window holds a
+    // transition into it.
+    for (uint32_t b = b0; b < b1; b += 4u) {
+        double qv[4], pv[4], d[4];
+        load4(q + b, qv);
+        load4(p + b, pv);
 #pragma unroll
-    for (int j = 0; j < kWinGroup; ++j) {
-        acc[j] = 0.0;
-        lo[j] = 1u;  // empty window
-        hi[j] = 0u;
-        wb[j] = 0;
-        if (j < nw) {
-            lo[j] = a.from[w0 + j];
-            hi[j] = a.to[w0 + j];
-            wb[j] = (long long)a.w_off[w0 + j] - (long long)lo[j];
+        for (int u = 0; u < 4; ++u) {
+            const double th = atan2(centred(pv[u], a.means, mp), centred(qv[u], a.means, mq));
+            d[u] = Rn::sub(th, prev);
+            if (d[u] < 0.0) d[u] = Rn::add(d[u], 2.0 * M_PI);
+            prev = th;
         }
-    }
-    const size_t row = i * a.S;  // this particle's samples
-    double prev = atan2(centred(p[row + s0], a.means, mp), centred(q[row + s0], a.means, mq));
-    for (uint32_t s = s0; s < s1; ++s) {
-        const size_t o = row + s + 1u;
-        const double th = atan2(centred(p[o], a.means, mp), centred(q[o], a.means, mq));
-        double d = Rn::sub(th, prev);
-        if (d < 0.0) d = Rn::add(d, 2.0 * M_PI);
-        prev = th;
 #pragma unroll
-        for (int j = 0; j < kWinGroup; ++j)
-            if (s >= lo[j] && s < hi[j]) acc[j] = Rn::add(acc[j], Rn::mul(a.w[wb[j] + s], d));
+        for (int j = 0; j < kWinGroup; ++j) {
+            if (j >= nw) break;
+            const Window v = win[j];
+            if (b > v.last || b + 3u < v.first) continue;
+            if (b >= v.first && b + 3u <= v.last) {
+#pragma unroll
+                for (int u = 0; u < 4; ++u) acc[j] = Rn::add(acc[j], Rn::mul(v.w[b + u], d[u]));
+            } else {
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    if (b + u >= v.first && b + u <= v.last)
+                        acc[j] = Rn::add(acc[j], Rn::mul(v.w[b + u], d[u]));
+            }
+        }
     }
 #pragma unroll
     for (int j = 0; j < kWinGroup; ++j)
@@ -264,7 +363,7 @@ __global__ void __launch_bounds__(256) fft_gather2_kernel(const double *x, const
                                                           const double *means, size_t n,
                                                           uint32_t from, uint32_t len,
                                                           const double *h, double2 *z, size_t S,
-                                                          int plane) {
+                                                          size_t pitch, int plane) {
     const size_t t = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (t >= n * len) return;
     const size_t i = t / len;
@@ -272,7 +371,7 @@ __global__ void __launch_bounds__(256) fft_gather2_kernel(const double *x, const
     const double *q = plane ? y : x, *p = plane ? py : px;
     const double mq = mean_of(means, n, i, 2 * plane, S);
     const double mp = mean_of(means, n, i, 2 * plane + 1, S);
-    const size_t o = i * S + from + k;
+    const size_t o = i * pitch + from + k;
     const double re = centred(q[o], means, mq), im = centred(p[o], means, mp);
     const double hk = h[k];
     z[(size_t(plane) * n + i) * len + k] = make_double2(re * hk, im * hk);
@@ -879,15 +978,14 @@ __global__ void __launch_bounds__(kFftThreadsMax) fft_tune_kernel(const FftTuneA
 }
 
 template <int ARITH, bool OCT>
-void launch_record_ok(const OrbitRecordArgs &a, unsigned blocks, int threads, cudaStream_t s) {
+void launch_record_ok(const OrbitRecordArgs &a, unsigned blocks, cudaStream_t s) {
     const bool kick = !isnan(a.kick_module);
-    const size_t smem = record_smem_bytes(threads);
     if (a.inverse) {
-        if (kick) orbit_record_kernel<ARITH, OCT, true, true><<<blocks, threads, smem, s>>>(a);
-        else orbit_record_kernel<ARITH, OCT, true, false><<<blocks, threads, smem, s>>>(a);
+        if (kick) orbit_record_kernel<ARITH, OCT, true, true><<<blocks, 64, 0, s>>>(a);
+        else orbit_record_kernel<ARITH, OCT, true, false><<<blocks, 64, 0, s>>>(a);
     } else {
-        if (kick) orbit_record_kernel<ARITH, OCT, false, true><<<blocks, threads, smem, s>>>(a);
-        else orbit_record_kernel<ARITH, OCT, false, false><<<blocks, threads, smem, s>>>(a);
+        if (kick) orbit_record_kernel<ARITH, OCT, false, true><<<blocks, 64, 0, s>>>(a);
+        else orbit_record_kernel<ARITH, OCT, false, false><<<blocks, 64, 0, s>>>(a);
     }
 }
 
@@ -895,18 +993,16 @@ void launch_record_ok(const OrbitRecordArgs &a, unsigned blocks, int threads, cu
 
 cudaError_t launch_orbit_record(const OrbitRecordArgs &a, cudaStream_t s) {
     if (a.n == 0) return cudaSuccess;
-    // One warp per block: the orbit of few particles is a long serial chain,
-    // spread over as many SMs as possible, and the staging buffer (17 KB a
-    // warp) sets the residency, not the block size.
-    const int threads = 32;
-    const unsigned blocks = unsigned((a.n + threads - 1) / threads);
+    // 32 particles per block: the orbits of few particles are spread over as
+    // many SMs as possible.
+    const unsigned blocks = unsigned((a.n + 31) / 32);
     const bool oct = a.mu != 0.0;
     if (a.arith == HM_ARITH_FAST) {
-        if (oct) launch_record_ok<HM_ARITH_FAST, true>(a, blocks, threads, s);
-        else launch_record_ok<HM_ARITH_FAST, false>(a, blocks, threads, s);
+        if (oct) launch_record_ok<HM_ARITH_FAST, true>(a, blocks, s);
+        else launch_record_ok<HM_ARITH_FAST, false>(a, blocks, s);
     } else {
-        if (oct) launch_record_ok<HM_ARITH_EXACT, true>(a, blocks, threads, s);
-        else launch_record_ok<HM_ARITH_EXACT, false>(a, blocks, threads, s);
+        if (oct) launch_record_ok<HM_ARITH_EXACT, true>(a, blocks, s);
+        else launch_record_ok<HM_ARITH_EXACT, false>(a, blocks, s);
     }
     return cudaGetLastError();
 }
@@ -932,11 +1028,12 @@ cudaError_t launch_hann_table(double *h, uint32_t len, cudaStream_t s) {
 cudaError_t launch_fft_gather2(const double *x, const double *px, const double *y,
                                const double *py, const double *means, size_t n, uint32_t from,
                                uint32_t len, const double *h, double2 *z, size_t S,
-                               cudaStream_t s) {
+                               size_t pitch, cudaStream_t s) {
     if (n == 0 || len == 0) return cudaSuccess;
     const unsigned grid = unsigned((n * len + 255) / 256);
     for (int plane = 0; plane < 2; ++plane) {
-        fft_gather2_kernel<<<grid, 256, 0, s>>>(x, px, y, py, means, n, from, len, h, z, S, plane);
+        fft_gather2_kernel<<<grid, 256, 0, s>>>(x, px, y, py, means, n, from, len, h, z, S, pitch,
+                                                plane);
         const cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }

@@ -367,3 +367,30 @@ def test_tracker_megno_inverse_matches_oracle(gpu):
         m = ~np.isnan(b)
         np.testing.assert_allclose(a[m], b[m], rtol=1e-12, atol=1e-14)
     assert np.isfinite(got[:, 1]).any()
+
+
+@pytest.mark.parametrize("n_turns", [1, 14, 15, 16, 17, 31, 64, 65, 130])
+@pytest.mark.parametrize("n", [1, 32, 33])
+def test_orbit_groups_and_segments(gpu, n, n_turns):
+    # Orbits around the 16-sample groups they are recorded in and the
+    # segments of the Birkhoff sums: lost particles, one with a single NaN
+    # coordinate, windows of one and two samples and odd bounds.
+    rng = np.random.default_rng(n + n_turns)
+    c = [rng.normal(0, 0.4, n) for _ in range(4)]
+    if n > 2:
+        c[0][1] = np.nan
+    frm = [0, n_turns // 3, n_turns - 1, n_turns // 2]
+    to = [n_turns, (2 * n_turns + 2) // 3, n_turns, n_turns // 2]
+    tabs = O.tables(n_turns, *TUNES, "sps", epsilon=16.0)
+    tr = C.Tracker(n_turns, *TUNES, "sps", NAN, 16.0, 0)
+    p = C.Particles(*c)
+    b, _ = C.tracker_orbit_tunes(tr, p, n_turns, 0.2, 10.0, frm, to, False, False)
+    orb = T.orbit(*c, tabs, n_turns, 0.2)
+    want = np.array([T.tune_vec(*(orb[k, :, i] for k in range(4)), frm, to, "birkhoff")
+                     for i in range(n)])
+    _close(b, want, 1e-13, "birkhoff")
+    got = p.state()
+    ref = O.track(*c, np.zeros(n, np.uint32), tabs, n_turns, 0.2, 10.0)
+    for k in range(4):
+        assert_bitwise(got[k], ref[k], f"coordinate {k}")
+    np.testing.assert_array_equal(got[4], ref[4])
