@@ -347,10 +347,10 @@ class henon_tracker:
                       inverse=False, from_idx=np.array([]), to_idx=np.array([])):
         import pandas as pd
 
-        result = np.asarray(self.tracker.birkhoff_tunes(
+        result, _ = self.tracker._window_tunes(
             particles.particles, n_turns, mu, barrier, kick_module, inverse,
             [int(v) for v in np.asarray(from_idx).ravel()],
-            [int(v) for v in np.asarray(to_idx).ravel()]))
+            [int(v) for v in np.asarray(to_idx).ravel()], False)
         pd_result = pd.DataFrame(columns=["from", "to", "tune_x", "tune_y"])
         for i in range(len(from_idx)):
             pd_result.loc[i] = [from_idx[i], to_idx[i], result[:, i * 2], result[:, i * 2 + 1]]
@@ -361,10 +361,10 @@ class henon_tracker:
                  from_idx=np.array([]), to_idx=np.array([])):
         import pandas as pd
 
-        result_birkhoff, result_fft = (np.asarray(r) for r in self.tracker.all_tunes(
+        result_birkhoff, result_fft = self.tracker._window_tunes(
             particles.particles, n_turns, mu, barrier, kick_module, inverse,
             [int(v) for v in np.asarray(from_idx).ravel()],
-            [int(v) for v in np.asarray(to_idx).ravel()]))
+            [int(v) for v in np.asarray(to_idx).ravel()], True)
         pd_result = pd.DataFrame(columns=["from", "to", "tune_x_birkhoff", "tune_y_birkhoff",
                                           "tune_x_fft", "tune_y_fft"])
         for i in range(len(from_idx)):

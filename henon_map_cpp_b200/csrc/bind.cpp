@@ -569,6 +569,27 @@ class storage_4d(_CpuClassNotProvided):
         }, py::arg("particles"), py::arg("n_turns"), py::arg("mu"), py::arg("barrier") = 100.0,
            py::arg("kick_module") = NAN, py::arg("inverse") = false,
            py::arg("from_idx") = std::vector<uint32_t>(), py::arg("to_idx") = std::vector<uint32_t>())
+        // The caller's windows and the full orbit alone, without the window
+        // [0, n_turns] that birkhoff_tunes and all_tunes append: what the
+        // facade's tables show.  fft: mean removed, both estimates (as
+        // all_tunes), else the Birkhoff tunes (as birkhoff_tunes).
+        .def("_window_tunes", [](Tracker &t, Particles &p, unsigned n_turns, double mu,
+                                 double barrier, double kick, bool inverse,
+                                 std::vector<uint32_t> from, std::vector<uint32_t> to, bool fft) {
+            if (from.size() != to.size())
+                throw std::runtime_error("compute_tune: from and to must be of the same size");
+            auto b = array2(p.n_total(), 2 * (from.size() + 1));
+            auto f = array2(fft ? p.n_total() : 0, 2 * (from.size() + 1));
+            hm_status s;
+            {
+                py::gil_scoped_release nogil;
+                s = hm_tracker_orbit_tunes(t.h, p.h, n_turns, mu, barrier, kick, inverse ? 1 : 0,
+                                           from.data(), to.data(), from.size(), fft ? 1 : 0,
+                                           b.mutable_data(), fft ? f.mutable_data() : nullptr);
+            }
+            check(s);
+            return py::make_tuple(b, f);
+        })
         .def("megno", [](Tracker &t, Particles &p, unsigned n_turns, double mu, double barrier,
                          double kick, bool inverse, std::vector<uint64_t> samples, int) {
             // Whole-orbit MEGNO (henon_tracker::megno, src/henon.cu:2755-2887)
