@@ -266,9 +266,8 @@ cudaError_t launch_fp64_peak(double *sink, int blocks, int threads,
                              int iters, cudaStream_t s, double *flops);
 
 // Tangent-map and indicator kernels (tangent.cu).
-cudaError_t launch_matrices_step(double *M, const double *x, const double *px, const double *y,
-                                 const double *py, const double *table, uint32_t idx, double mu,
-                                 size_t n, bool set, cudaStream_t s);
+cudaError_t launch_matrices_step(double *M, const double *x, const double *y, const double *table,
+                                 uint32_t idx, double mu, size_t n, bool set, cudaStream_t s);
 cudaError_t launch_matrices_identity(double *M, size_t n, cudaStream_t s);
 cudaError_t launch_matrices_apply(const double *M, const double *rv, double *out, size_t n,
                                   cudaStream_t s);

@@ -122,8 +122,7 @@ hm_status matrices_step(hm_matrices *m, const hm_tracker *t, const hm_particles 
     if (m->n && p->global_steps >= t->allowed_steps)
         return fail(HM_ERR_BUDGET,
                     "The number of turns is too large. (tangent matrix past the table end)");
-    HM_CUDA_TRY(hm::launch_matrices_step(m->m.as<double>(), p->x.as<double>(), p->px.as<double>(),
-                                         p->y.as<double>(), p->py.as<double>(),
+    HM_CUDA_TRY(hm::launch_matrices_step(m->m.as<double>(), p->x.as<double>(), p->y.as<double>(),
                                          t->table.as<double>(), p->global_steps, mu, m->n, set, 0));
     return ok();
 }
