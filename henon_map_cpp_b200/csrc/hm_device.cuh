@@ -255,8 +255,17 @@ __device__ __forceinline__ uint4 philox4x32_10(uint4 c, uint32_t k0, uint32_t k1
     return c;
 }
 
+// u = (int32(r) + 0.5) 2^-31, exactly: with r's sign bit flipped, u + 3 lies
+// in [2, 4) and has r's bits and a half behind them as its mantissa.
 __device__ __forceinline__ double kick_uniform(uint32_t r) {
-    return Rn::mul(Rn::add(double(int32_t(r)), 0.5), 0x1p-31);
+    const uint32_t b = r ^ 0x80000000u;
+    return Rn::sub(__hiloint2double(int(__funnelshift_r(b, 0x400u, 12)), int((b << 20) | 0x80000u)),
+                   3.0);
+}
+
+// s < 1 for s = u^2 + v^2, which is never NaN nor, as no u is 0, zero.
+__device__ __forceinline__ bool in_disc(double s) {
+    return static_cast<uint32_t>(__double2hiint(s)) < 0x3ff00000u;
 }
 
 struct KickDirection {
@@ -273,7 +282,7 @@ __device__ __forceinline__ KickDirection kick_direction(unsigned long long seed,
         if (!got1) {
             const double a1 = kick_uniform(r.x), a2 = kick_uniform(r.y);
             const double s = Rn::add(Rn::mul(a1, a1), Rn::mul(a2, a2));
-            if (s < 1.0) {
+            if (in_disc(s)) {
                 u1 = a1;
                 u2 = a2;
                 s1 = s;
@@ -283,7 +292,7 @@ __device__ __forceinline__ KickDirection kick_direction(unsigned long long seed,
         if (!got2) {
             const double a3 = kick_uniform(r.z), a4 = kick_uniform(r.w);
             const double s = Rn::add(Rn::mul(a3, a3), Rn::mul(a4, a4));
-            if (s < 1.0 && s > 0.0) {
+            if (in_disc(s)) {
                 u3 = a3;
                 u4 = a4;
                 s2 = s;

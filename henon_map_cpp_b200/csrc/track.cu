@@ -39,7 +39,7 @@ using dev::Turn;
 // with steps = the turns they survived.  A lost particle's registers are
 // set to zero, a fixed point of the map, so that it never trips the OR
 // again.
-template <int ARITH, bool OCT, bool REV, int K, bool KICK>
+template <int ARITH, bool OCT, bool REV, int K>
 __device__ __forceinline__ void turn_all(const TrackChunk &c, const Barrier &bar, double mu,
                                          const Turn &t, uint32_t k, Particle (&p)[K],
                                          const uint32_t (&id)[K], bool (&live)[K],
@@ -47,17 +47,8 @@ __device__ __forceinline__ void turn_all(const TrackChunk &c, const Barrier &bar
     uint32_t ored = 0u;
 #pragma unroll
     for (int j = 0; j < K; ++j) {
-        // Random kick: before the sextupole going forward (table index
-        // turn0 + k); going backward, subtracted after the inverse
-        // sextupole (table index turn0 - 1 - k), undoing the forward kick.
-        if (KICK && !REV)
-            dev::apply_kick<false>(p[j], dev::kick_direction(c.kick_seed, id[j], c.turn0 + k),
-                                   c.kick_module);
         dev::turn<ARITH, OCT, REV>(p[j], t, mu);
-        if (KICK && REV)
-            dev::apply_kick<true>(p[j], dev::kick_direction(c.kick_seed, id[j], c.turn0 - 1u - k),
-                                  c.kick_module);
-        if (!KICK || live[j]) ored |= dev::hi_or(p[j]);
+        ored |= dev::hi_or(p[j]);
     }
     if (__any_sync(kFullMask, !dev::small_or(ored, bar))) {
         const uint32_t s = REV ? c.turn0 - k : c.turn0 + k;
@@ -84,7 +75,7 @@ __device__ __forceinline__ void turn_all(const TrackChunk &c, const Barrier &bar
 // The chunk's turns with the turn records read from global memory: every
 // lane of a warp loads the same 32-byte record (one broadcast transaction,
 // an L1 hit after the first warp), prefetched one turn ahead.
-template <int ARITH, bool OCT, bool REV, int K, bool KICK>
+template <int ARITH, bool OCT, bool REV, int K>
 __device__ __forceinline__ void turns_direct(const TrackChunk &c, const Barrier &bar,
                                              Particle (&p)[K], const uint32_t (&id)[K],
                                              bool (&live)[K], bool warp_live) {
@@ -94,16 +85,16 @@ __device__ __forceinline__ void turns_direct(const TrackChunk &c, const Barrier 
     for (uint32_t k = 0; warp_live && k < nt; ++k) {
         const uint32_t kn = (k + 1 < nt) ? k + 1 : k;
         const Turn tn = dev::load_turn(c.table, REV ? c.turn0 - 1u - kn : c.turn0 + kn);
-        turn_all<ARITH, OCT, REV, K, KICK>(c, bar, mu, t, k, p, id, live, warp_live);
+        turn_all<ARITH, OCT, REV, K>(c, bar, mu, t, k, p, id, live, warp_live);
         t = tn;
     }
 }
 
-// Shared memory of a staged launch: two stage buffers of turn records and,
-// without kicks, two checkpoints {x, px, y, py} per particle.
+// Shared memory of a staged launch: two stage buffers of turn records and two
+// checkpoints {x, px, y, py} per particle.
 __host__ __device__ constexpr size_t staged_smem_bytes(uint32_t stage_turns, uint32_t threads,
-                                                       int per_thread, bool kick) {
-    return size_t(stage_turns) * 2u * 32u + (kick ? 0u : size_t(threads) * per_thread * 64u);
+                                                       int per_thread) {
+    return size_t(stage_turns) * 2u * 32u + size_t(threads) * per_thread * 64u;
 }
 
 __device__ __forceinline__ Turn staged_record(const double *rec, uint32_t kn, uint32_t kk,
@@ -121,7 +112,7 @@ __device__ __forceinline__ Turn staged_record(const double *rec, uint32_t kn, ui
 // broadcast.  Warps whose particles are all lost keep taking part in the
 // per-stage barriers; the block stops when none of its warps is live.
 //
-// Without kicks, a stage runs in blocks of turns with no per-turn control
+// A stage runs in blocks of turns with no per-turn control
 // flow (dev::block_turns): the thread saves its particles to shared memory
 // and applies the block's turns.  If the coordinates looked at stayed below
 // the bound, no particle can have been lost in the block, which is then
@@ -136,11 +127,11 @@ __device__ __forceinline__ Turn staged_record(const double *rec, uint32_t kn, ui
 // turns 4 % of the dynamic-aperture scan.
 // Returns false when a copy did not land within the bounded wait (the
 // chunk's results are then invalid and c.fault is set).
-template <int ARITH, bool OCT, bool REV, int K, bool KICK>
+template <int ARITH, bool OCT, bool REV, int K>
 __device__ __forceinline__ bool turns_staged(const TrackChunk &c, const Barrier &bar,
                                              Particle (&p)[K], const uint32_t (&id)[K],
                                              bool (&live)[K], bool warp_live) {
-    // [2][S][4] turn records, then (no kicks) [K][blockDim.x] checkpoints.
+    // [2][S][4] turn records, then [2][K][blockDim.x] checkpoints.
     extern __shared__ __align__(128) double stage_buf[];
     __shared__ __align__(8) uint64_t full[2];
     const double mu = c.mu;
@@ -183,12 +174,7 @@ __device__ __forceinline__ bool turns_staged(const TrackChunk &c, const Barrier 
         const uint32_t k0 = st * S;
         const uint32_t kn = min(S, nt - k0);
         const double *rec = stage_buf + size_t(buf) * S * 4u;
-        if (!timed_out && KICK) {
-#pragma unroll 2
-            for (uint32_t kk = 0; warp_live && kk < kn; ++kk)
-                turn_all<ARITH, OCT, REV, K, KICK>(c, bar, mu, staged_record(rec, kn, kk, REV),
-                                                   k0 + kk, p, id, live, warp_live);
-        } else if (!timed_out) {
+        if (!timed_out) {
             // A caller's records are checked to be rotations, which the
             // test of every second turn needs.
             bool pairs = c.pair_hi != 0u;
@@ -254,9 +240,8 @@ __device__ __forceinline__ bool turns_staged(const TrackChunk &c, const Barrier 
                     }
                     const uint32_t j1 = min(j0, kn);
                     for (uint32_t kk = j0 - B; warp_live && kk < j1; ++kk)
-                        turn_all<ARITH, OCT, REV, K, KICK>(c, bar, mu,
-                                                           staged_record(rec, kn, kk, REV), k0 + kk,
-                                                           p, id, live, warp_live);
+                        turn_all<ARITH, OCT, REV, K>(c, bar, mu, staged_record(rec, kn, kk, REV),
+                                                     k0 + kk, p, id, live, warp_live);
                     check = false;
                 }
             }
@@ -283,6 +268,182 @@ __device__ __forceinline__ bool turns_staged(const TrackChunk &c, const Barrier 
     const bool fault = __syncthreads_or(timed_out);
     if (fault && leader && c.fault) atomicOr(c.fault, 1u);
     return !fault;
+}
+
+// ---- kicked turns --------------------------------------------------------------
+// The kicks do not depend on the orbit, so a warp makes those of kKickTurns
+// turns of its 32 particles together and then runs the turns.  Each kick
+// takes the first point of each of two attempts' sequences that lies in the
+// unit disc (dev::kick_direction), 1.6 Philox blocks on average; with the
+// rejection loop inside the turn a warp waited for its slowest lane, 3.6
+// blocks a turn.  Here every lane makes the first attempt of its own kicks,
+// the rejected ones (38 %) go to a list, and each further attempt is made for
+// the whole list by full warps: 1.9 blocks a turn.
+//
+// 262,144 particles x 2,000 turns, mu = 0.2: 10.0 ms before, 6.4 now, 66 % of
+// the issue slots and 37 % of the FP64 pipe busy; 299 instructions per warp
+// and turn (421 before), about half of them the generator's.  Groups of 4
+// turns 7.5 ms, of 16 6.8 (fewer warps fit).
+//
+// Shared memory of a warp: the points (then the kicks) of its turns, the list,
+// the particles' indices and the turns' records.
+constexpr uint32_t kKickTurns = 8;
+
+struct KickShared {
+    double2 a[kKickTurns * 32], b[kKickTurns * 32];  // {u1, u2}, {u3, u4} of [turn][lane]
+    double2 rec[2 * kKickTurns];
+    uint16_t list[kKickTurns * 32];
+    uint32_t id[32];
+};
+
+// One attempt at the kick of (turn, id): keeps the point of each disc that
+// has none yet; `got` holds bit 0 (first disc) and bit 1.
+__device__ __forceinline__ uint32_t kick_attempt(uint32_t k0, uint32_t k1, uint32_t id,
+                                                 uint32_t turn, uint32_t attempt, uint32_t got,
+                                                 double2 *a, double2 *b) {
+    const uint4 r = dev::philox4x32_10(make_uint4(turn, attempt, id, 0u), k0, k1);
+    const double a1 = dev::kick_uniform(r.x), a2 = dev::kick_uniform(r.y);
+    const double a3 = dev::kick_uniform(r.z), a4 = dev::kick_uniform(r.w);
+    const bool in1 = dev::in_disc(Rn::add(Rn::mul(a1, a1), Rn::mul(a2, a2)));
+    const bool in2 = dev::in_disc(Rn::add(Rn::mul(a3, a3), Rn::mul(a4, a4)));
+    if (in1 && !(got & 1u)) *a = make_double2(a1, a2);
+    if (in2 && !(got & 2u)) *b = make_double2(a3, a4);
+    return got | (in1 ? 1u : 0u) | (in2 ? 2u : 0u);
+}
+
+// The kicks (direction times module) of the turns with table indices
+// t0, t0 + dt, ... (kn of them) of the warp's live particles.
+__device__ __forceinline__ void make_kicks(KickShared &w, const TrackChunk &c, uint32_t id,
+                                           bool live, uint32_t t0, int dt, uint32_t kn) {
+    const unsigned lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
+    const uint32_t k0 = uint32_t(c.kick_seed), k1 = uint32_t(c.kick_seed >> 32);
+    uint32_t n_list = 0;
+#pragma unroll 4
+    for (uint32_t u = 0; u < kKickTurns; ++u) {
+        const uint32_t slot = u * 32u + lane;
+        // what kick_direction falls back to when no attempt gives a point
+        w.a[slot] = make_double2(0.0, 0.0);
+        w.b[slot] = make_double2(1.0, 0.0);
+        const uint32_t got =
+            kick_attempt(k0, k1, id, t0 + uint32_t(int(u) * dt), 0u, 0u, &w.a[slot], &w.b[slot]);
+        const bool more = live && u < kn && got != 3u;
+        const unsigned m = __ballot_sync(kFullMask, more);
+        if (more) w.list[n_list + __popc(m & below)] = uint16_t(slot | (got << 14));
+        n_list += __popc(m);
+    }
+    for (uint32_t at = 1; n_list > 0u && at < dev::kKickAttempts; ++at) {
+        __syncwarp();
+        uint32_t left = 0;
+        for (uint32_t base = 0; base < n_list; base += 32u) {
+            const bool mine = base + lane < n_list;
+            uint32_t e = mine ? w.list[base + lane] : 0u;
+            __syncwarp();  // read before the entries kept are written over it
+            bool more = false;
+            if (mine) {
+                const uint32_t slot = e & 0x3fffu;
+                const uint32_t got = kick_attempt(k0, k1, w.id[slot & 31u],
+                                                  t0 + uint32_t(int(slot >> 5) * dt), at, e >> 14,
+                                                  &w.a[slot], &w.b[slot]);
+                more = got != 3u;
+                e = slot | (got << 14);
+            }
+            const unsigned m = __ballot_sync(kFullMask, more);
+            if (more) w.list[left + __popc(m & below)] = uint16_t(e);
+            left += __popc(m);
+        }
+        n_list = left;
+    }
+    __syncwarp();
+    // (u1, u2, u3 f, u4 f), f = sqrt((1 - s1) / s2), times the module
+    const double km = c.kick_module;
+#pragma unroll 4
+    for (uint32_t u = 0; u < kKickTurns; ++u) {
+        const double2 a = w.a[u * 32u + lane], b = w.b[u * 32u + lane];
+        const double s1 = Rn::add(Rn::mul(a.x, a.x), Rn::mul(a.y, a.y));
+        const double s2 = Rn::add(Rn::mul(b.x, b.x), Rn::mul(b.y, b.y));
+        const double f = __dsqrt_rn(Rn::div(Rn::sub(1.0, s1), s2));
+        w.a[u * 32u + lane] = make_double2(Rn::mul(a.x, km), Rn::mul(a.y, km));
+        w.b[u * 32u + lane] = make_double2(Rn::mul(Rn::mul(b.x, f), km), Rn::mul(Rn::mul(b.y, f), km));
+    }
+}
+
+// Adds (forward) or subtracts (backward) a kick and refreshes the squares.
+template <bool SUB>
+__device__ __forceinline__ void add_kick(Particle &p, double2 a, double2 b) {
+    if (SUB) {
+        p = dev::make_particle(Rn::sub(p.x, a.x), Rn::sub(p.px, a.y), Rn::sub(p.y, b.x),
+                               Rn::sub(p.py, b.y));
+    } else {
+        p = dev::make_particle(Rn::add(p.x, a.x), Rn::add(p.px, a.y), Rn::add(p.y, b.x),
+                               Rn::add(p.py, b.y));
+    }
+}
+
+// The chunk's turns with kicks (one particle per thread): groups of
+// kKickTurns turns, redone with the per-turn test where a live particle's
+// coordinate reached the bound.  A lost particle's registers move with the
+// kicks of its slot; nothing reads them.
+template <int ARITH, bool OCT, bool REV>
+__device__ __forceinline__ void turns_kicked(const TrackChunk &c, const Barrier &bar,
+                                             Particle &p, uint32_t id, bool &live,
+                                             bool warp_live) {
+    extern __shared__ __align__(128) double stage_buf[];
+    KickShared &w = reinterpret_cast<KickShared *>(stage_buf)[threadIdx.x >> 5];
+    const unsigned lane = threadIdx.x & 31u;
+    const double mu = c.mu;
+    w.id[lane] = id;
+    auto turn = [&](uint32_t u) {
+        const double2 a = w.a[u * 32u + lane], b = w.b[u * 32u + lane];
+        const double2 r = w.rec[2u * u], t = w.rec[2u * u + 1u];
+        if (!REV) add_kick<false>(p, a, b);
+        dev::turn<ARITH, OCT, REV>(p, Turn{r.x, r.y, t.x, t.y}, mu);
+        if (REV) add_kick<true>(p, a, b);
+    };
+    for (uint32_t k0 = 0; warp_live && k0 < c.n_turns; k0 += kKickTurns) {
+        const uint32_t kn = min(kKickTurns, c.n_turns - k0);
+        const uint32_t t0 = REV ? c.turn0 - 1u - k0 : c.turn0 + k0;
+        if (lane < 2u * kn) {  // half `lane & 1` of the record of turn lane / 2
+            const uint32_t t = REV ? t0 - (lane >> 1) : t0 + (lane >> 1);
+            w.rec[lane] = __ldg(reinterpret_cast<const double2 *>(c.table) + 2u * size_t(t) +
+                                (lane & 1u));
+        }
+        __syncwarp();
+        make_kicks(w, c, id, live, t0, REV ? -1 : 1, kn);
+        __syncwarp();
+        const Particle from = p;
+        float big = 0.0f;
+        auto look = [&]() { big = dev::hi_max(dev::hi_max(big, p.x, p.px), p.y, p.py); };
+        if (kn == kKickTurns) {
+#pragma unroll
+            for (uint32_t u = 0; u < kKickTurns; ++u) {
+                turn(u);
+                look();
+            }
+        } else {
+            for (uint32_t u = 0; u < kn; ++u) {
+                turn(u);
+                look();
+            }
+        }
+        const bool over = live && (__float_as_uint(big) & 0x7fffffffu) >= bar.small_hi;
+        if (__any_sync(kFullMask, over)) {
+            p = from;
+            for (uint32_t u = 0; u < kn; ++u) {
+                turn(u);
+                if (live && !dev::inside_after_turn<ARITH>(p, bar)) {
+                    c.ux[id] = quiet_nan();
+                    c.upx[id] = quiet_nan();
+                    c.uy[id] = quiet_nan();
+                    c.upy[id] = quiet_nan();
+                    c.usteps[id] = REV ? c.turn0 - k0 - u : c.turn0 + k0 + u;
+                    live = false;
+                }
+            }
+            warp_live = __any_sync(kFullMask, live);
+        }
+        if (!live) p = dev::make_particle(0.0, 0.0, 0.0, 0.0);
+        __syncwarp();
+    }
 }
 
 // One chunk of turns for the particles of one block (K per thread).
@@ -328,10 +489,13 @@ __device__ __forceinline__ void track_chunk(const TrackChunk &c) {
 #pragma unroll
     for (int j = 0; j < K; ++j) thread_live |= live[j];
     const bool warp_live = __any_sync(kFullMask, thread_live);
-    if (STAGED) {
-        if (!turns_staged<ARITH, OCT, REV, K, KICK>(c, bar, p, id, live, warp_live)) return;
+    if constexpr (KICK) {
+        static_assert(K == 1, "kicked turns run one particle per thread");
+        turns_kicked<ARITH, OCT, REV>(c, bar, p[0], id[0], live[0], warp_live);
+    } else if (STAGED) {
+        if (!turns_staged<ARITH, OCT, REV, K>(c, bar, p, id, live, warp_live)) return;
     } else {
-        turns_direct<ARITH, OCT, REV, K, KICK>(c, bar, p, id, live, warp_live);
+        turns_direct<ARITH, OCT, REV, K>(c, bar, p, id, live, warp_live);
     }
 
     if (c.out_idx == nullptr) {
@@ -381,26 +545,35 @@ __device__ __forceinline__ void track_chunk(const TrackChunk &c) {
 //     exact, mu != 0     80.7  74.8  72.7  71.6   (before: 91.9  79.9  76.4  74.6)
 // Before: per-turn looks, runs of 32 turns, 64 registers.  With 64 registers
 // the blocks of turns took 68.3, 48.8, 47.1 and 44.9 at mu = 0.
-template <int ARITH, bool OCT, bool REV, int K, bool STAGED, bool KICK>
+template <int ARITH, bool OCT, bool REV, int K, bool STAGED>
 __global__ void __launch_bounds__(256, K <= 2 ? 2 : 1) track_chunk_kernel(const TrackChunk c) {
-    track_chunk<ARITH, OCT, REV, K, STAGED, KICK>(c);
+    track_chunk<ARITH, OCT, REV, K, STAGED, false>(c);
 }
 
-template <int ARITH, bool OCT, bool REV, int K, bool KICK>
+// 80 registers: six blocks of 128 threads, as many as the shared memory holds
+// (with 96, five: 6.74 against 6.40 ms).
+template <int ARITH, bool OCT, bool REV>
+__global__ void __launch_bounds__(256, 3) track_kicked_kernel(const TrackChunk c) {
+    track_chunk<ARITH, OCT, REV, 1, false, true>(c);
+}
+
+// Dynamic plus static shared memory above 48 KB needs the opt-in (the
+// staged kernels' static part is their two mbarriers).
+template <class Kernel>
+cudaError_t allow_smem(Kernel kernel, size_t smem) {
+    if (smem <= 40u * 1024u) return cudaSuccess;
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+}
+
+template <int ARITH, bool OCT, bool REV, int K>
 cudaError_t launch_s(const TrackChunk &c, unsigned blocks, int threads, cudaStream_t s) {
     if (c.stage_turns == 0) {
-        track_chunk_kernel<ARITH, OCT, REV, K, false, KICK><<<blocks, threads, 0, s>>>(c);
+        track_chunk_kernel<ARITH, OCT, REV, K, false><<<blocks, threads, 0, s>>>(c);
     } else {
-        const size_t smem = staged_smem_bytes(c.stage_turns, uint32_t(threads), K, KICK);
-        auto kernel = track_chunk_kernel<ARITH, OCT, REV, K, true, KICK>;
-        // Dynamic plus static shared memory above 48 KB needs the opt-in
-        // (the kernel's static part is its two mbarriers): 256 threads with
-        // four particles each and 256-turn stages take exactly 48 KB dynamic.
-        if (smem > 40u * 1024u) {
-            const cudaError_t e =
-                cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-            if (e != cudaSuccess) return e;
-        }
+        const size_t smem = staged_smem_bytes(c.stage_turns, uint32_t(threads), K);
+        auto kernel = track_chunk_kernel<ARITH, OCT, REV, K, true>;
+        const cudaError_t e = allow_smem(kernel, smem);
+        if (e != cudaSuccess) return e;
         kernel<<<blocks, threads, smem, s>>>(c);
     }
     return cudaGetLastError();
@@ -428,11 +601,14 @@ cudaError_t launch_k(const TrackChunk &c, const TrackLaunch &l, uint32_t n_upper
                      cudaStream_t s) {
     int threads = l.threads;
     if (!isnan(c.kick_module)) {
-        // Kicked turns are dominated by the integer work of the generator:
-        // one particle per thread.
         const unsigned blocks = unsigned((uint64_t(n_upper) + threads - 1) / threads);
         if (blocks == 0) return cudaSuccess;
-        return launch_s<ARITH, OCT, REV, 1, true>(c, blocks, threads, s);
+        const size_t smem = size_t(threads / 32) * sizeof(KickShared);
+        auto kernel = track_kicked_kernel<ARITH, OCT, REV>;
+        const cudaError_t e = allow_smem(kernel, smem);
+        if (e != cudaSuccess) return e;
+        kernel<<<blocks, threads, smem, s>>>(c);
+        return cudaGetLastError();
     }
     // Several particles per thread add instruction-level parallelism once
     // the device is full; a short list would instead leave SMs idle (a
@@ -452,9 +628,9 @@ cudaError_t launch_k(const TrackChunk &c, const TrackLaunch &l, uint32_t n_upper
     const unsigned blocks = unsigned((uint64_t(n_upper) + per_block - 1) / per_block);
     if (blocks == 0) return cudaSuccess;
     switch (K) {
-        case 1: return launch_s<ARITH, OCT, REV, 1, false>(c, blocks, threads, s);
-        case 2: return launch_s<ARITH, OCT, REV, 2, false>(c, blocks, threads, s);
-        case 4: return launch_s<ARITH, OCT, REV, 4, false>(c, blocks, threads, s);
+        case 1: return launch_s<ARITH, OCT, REV, 1>(c, blocks, threads, s);
+        case 2: return launch_s<ARITH, OCT, REV, 2>(c, blocks, threads, s);
+        case 4: return launch_s<ARITH, OCT, REV, 4>(c, blocks, threads, s);
         default: return cudaErrorInvalidValue;
     }
 }

@@ -87,3 +87,27 @@ def test_device_tables_that_are_not_rotations(gpu, scale):
            n_turns, 0, n_turns, 0.0, 10.0, 0, 0, ws.data_ptr(), None)
     check([d.cpu().numpy() for d in dev] + [steps.cpu().numpy().view(np.uint32)], want,
           f"scale {scale}")
+
+
+@pytest.mark.parametrize("inverse", [False, True])
+@pytest.mark.parametrize("n_turns", [1, 7, 8, 9, 100])
+@pytest.mark.parametrize("n", [1, 31, 33, 300])
+def test_kicked_groups_of_turns(gpu, n, n_turns, inverse):
+    # Kicks are made for groups of 8 turns, rejected points by whole warps:
+    # part groups, part warps, losses inside a group, a set that starts
+    # with NaN particles, both directions.
+    c = points(n, 0.6, 11)
+    if n > 2:
+        c[2][n // 2] = np.nan
+    seed, kick, mu = 0x9E3779B97F4A7C15, 0.02, 0.2
+    tabs = O.tables(max(n_turns, 1), *TUNES, "sps", epsilon=16.0)
+    t = C.Tracker(n_turns, *TUNES, "sps", NAN, 16.0, 0)
+    p = C.Particles(*c)
+    p.kick_seed = seed
+    want = (*c, np.zeros(n, np.uint32))
+    if inverse:
+        want = O.track(*want, tabs, n_turns, mu, 10.0)
+        t.track(p, n_turns, mu, 10.0)
+    want = O.track_kicked(*want, tabs, n_turns, mu, 10.0, kick, seed, inverse=inverse)
+    t.track(p, n_turns, mu, 10.0, kick, inverse)
+    check(p.state(), want, "kicked")
