@@ -95,9 +95,17 @@ __device__ __forceinline__ uint64_t next_sample(const uint64_t *turns, int n, ui
 // holds about half of a particle's window accumulators, so the same shared
 // memory holds twice the threads: the loop is a long chain of dependent
 // FP64 operations, and more warps per SM hide its latency.
+// PLANES: the tunes' y plane goes to the even warp.  The warp that finishes
+// last decides, and which one that is depends on the windows: with many open
+// the vector warp's two angles and window sums outlast the matrix work.
+// 65,025 particles, 13 windows of 100 .. 10^4 turns, ms for the first 4096
+// turns (5.4 of 13 windows open on average), the next (2.8) and the last
+// 1808 (1.5): 31.1, 20.3, 8.4 with both planes in the vector warp, 27.5, 21.1,
+// 9.3 with one in each.  launch_oct splits above kPlanesOpen.
 // EXT: kicks and backward turns (whole-orbit MEGNO: DO_M alone, the
 // Jacobian of each turn at the point before it).
-template <bool OCT, bool DO_M, bool DO_V, bool DO_T, bool SPLIT, bool EXT = false>
+template <bool OCT, bool DO_M, bool DO_V, bool DO_T, bool SPLIT, bool EXT = false,
+          bool PLANES = false>
 __global__ void __launch_bounds__(128, SPLIT ? 4 : 1) indicators_kernel(const FusedArgs a) {
     extern __shared__ double smem[];
     const unsigned warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
@@ -105,7 +113,8 @@ __global__ void __launch_bounds__(128, SPLIT ? 4 : 1) indicators_kernel(const Fu
     // warps the vector and tune work; without it, every warp does all.
     const bool role_m = !SPLIT || (warp & 1u) == 0u;
     const bool role_v = !SPLIT || (warp & 1u) == 1u;
-    const bool do_m = DO_M && role_m, do_v = DO_V && role_v, do_t = DO_T && role_v;
+    const bool do_m = DO_M && role_m, do_v = DO_V && role_v;
+    const bool do_tx = DO_T && role_v, do_ty = DO_T && (PLANES ? role_m : role_v);
     // Threads (per role) of a block, and this thread's index among them.
     const int T = SPLIT ? int(blockDim.x) / 2 : int(blockDim.x);
     const int tid = SPLIT ? int((warp >> 1) * 32u + lane) : int(threadIdx.x);
@@ -162,21 +171,24 @@ __global__ void __launch_bounds__(128, SPLIT ? 4 : 1) indicators_kernel(const Fu
         }
     }
     double store_x = 0.0, store_y = 0.0;
-    if (do_t) {
-        store_x = a.store_x[ii];
-        store_y = a.store_y[ii];
+    if (do_tx) store_x = a.store_x[ii];
+    if (do_ty) store_y = a.store_y[ii];
+    if (DO_T)
         for (int w = 0; w < a.n_tu; ++w) {
             const size_t g = size_t(tab_tu[w].orig) * n + ii;
-            t1x[w * T + tid] = a.t1x[g];
-            t1y[w * T + tid] = a.t1y[g];
-            t2x[w * T + tid] = a.t2x[g];
-            t2y[w * T + tid] = a.t2y[g];
+            if (do_tx) {
+                t1x[w * T + tid] = a.t1x[g];
+                t2x[w * T + tid] = a.t2x[g];
+            }
+            if (do_ty) {
+                t1y[w * T + tid] = a.t1y[g];
+                t2y[w * T + tid] = a.t2y[g];
+            }
         }
-    }
 
     const double mu = a.mu;
     const dev::Barrier bar = dev::make_barrier<HM_ARITH_EXACT>(a.b2bits);
-    bool warp_live = __any_sync(dev::kFullMask, alive);
+    const bool warp_live = __any_sync(dev::kFullMask, alive);
     // First open window of each kind, and the next MEGNO sample turn.
     const bool snaps = do_m && a.megno_l1 && a.n_snap > 0;
     uint64_t next_snap = snaps ? next_sample(a.snap_turns, a.n_snap, a.megno_idx) : ~0ull;
@@ -291,38 +303,70 @@ __global__ void __launch_bounds__(128, SPLIT ? 4 : 1) indicators_kernel(const Fu
                     ly_b[w * T + tid] = Rn::add(ly_b[w * T + tid], Rn::mul(l, e.w[idx]));
                 }
             }
+            // one reciprocal for the four quotients (dev::div_by)
+            const double inv = __drcp_rn(nv);
 #pragma unroll
-            for (int q = 0; q < 4; ++q) v[q] = Rn::div(t4[q], nv);
-        }
-        if (do_t) {
-            const double ax = atan2(px, x), ay = atan2(py, y);
-            double dx = Rn::sub(ax, store_x), dy = Rn::sub(ay, store_y);
-            const double two_pi = 2 * M_PI;
-            dx = dx > 0 ? dx : Rn::add(dx, two_pi);
-            dy = dy > 0 ? dy : Rn::add(dy, two_pi);
-            store_x = ax;
-            store_y = ay;
-            const uint64_t idx = a.tu_idx + k;
-            s_tu = first_open(tab_tu, a.n_tu, s_tu, idx);
-            for (int w = s_tu; w < a.n_tu; ++w) {
-                const WinEntry &e = tab_tu[w];
-                if (idx < e.len) {  // first window [0, T)
-                    const double wt = e.w[idx];
-                    t1x[w * T + tid] = Rn::add(t1x[w * T + tid], Rn::mul(dx, wt));
-                    t1y[w * T + tid] = Rn::add(t1y[w * T + tid], Rn::mul(dy, wt));
-                } else {  // second window [T, 2 T)
-                    const double wt = e.w[idx - e.len];
-                    t2x[w * T + tid] = Rn::add(t2x[w * T + tid], Rn::mul(dx, wt));
-                    t2y[w * T + tid] = Rn::add(t2y[w * T + tid], Rn::mul(dy, wt));
-                }
+            for (int q = 0; q < 4; ++q) v[q] = dev::div_by(t4[q], nv, inv);
+            if (dev::divisor_rare(nv) || dev::div_rare(t4[0]) || dev::div_rare(t4[1]) ||
+                dev::div_rare(t4[2]) || dev::div_rare(t4[3])) {
+#pragma unroll
+                for (int q = 0; q < 4; ++q) v[q] = Rn::div(t4[q], nv);
             }
         }
-        // A warp whose particles are all lost stops: every later update
-        // would only add NaN to windows that are still open (fixed below).
-        if (!alive) warp_live = __any_sync(dev::kFullMask, alive);
+        if (DO_T) {
+            const double two_pi = 2 * M_PI;
+            const uint64_t idx = a.tu_idx + k;
+            if (do_tx || do_ty) s_tu = first_open(tab_tu, a.n_tu, s_tu, idx);
+            auto plane = [&](double q, double p, double &store, double *t1, double *t2) {
+                const double an = atan2(p, q);
+                double d = Rn::sub(an, store);
+                d = d > 0 ? d : Rn::add(d, two_pi);
+                store = an;
+                for (int w = s_tu; w < a.n_tu; ++w) {
+                    const WinEntry &e = tab_tu[w];
+                    const bool one = idx < e.len;  // first window [0, T), else second [T, 2 T)
+                    const double wt = e.w[one ? idx : idx - e.len];
+                    double &acc = (one ? t1 : t2)[w * T + tid];
+                    acc = Rn::add(acc, Rn::mul(d, wt));
+                }
+            };
+            auto both = [&]() {
+                const double ax = atan2(px, x), ay = atan2(py, y);
+                double dx = Rn::sub(ax, store_x), dy = Rn::sub(ay, store_y);
+                dx = dx > 0 ? dx : Rn::add(dx, two_pi);
+                dy = dy > 0 ? dy : Rn::add(dy, two_pi);
+                store_x = ax;
+                store_y = ay;
+                for (int w = s_tu; w < a.n_tu; ++w) {
+                    const WinEntry &e = tab_tu[w];
+                    if (idx < e.len) {  // first window [0, T)
+                        const double wt = e.w[idx];
+                        t1x[w * T + tid] = Rn::add(t1x[w * T + tid], Rn::mul(dx, wt));
+                        t1y[w * T + tid] = Rn::add(t1y[w * T + tid], Rn::mul(dy, wt));
+                    } else {  // second window [T, 2 T)
+                        const double wt = e.w[idx - e.len];
+                        t2x[w * T + tid] = Rn::add(t2x[w * T + tid], Rn::mul(dx, wt));
+                        t2y[w * T + tid] = Rn::add(t2y[w * T + tid], Rn::mul(dy, wt));
+                    }
+                }
+            };
+            if (PLANES) {
+                if (role_v) plane(x, px, store_x, t1x, t2x);
+                else plane(y, py, store_y, t1y, t2y);
+            } else if (role_v) {
+                both();
+            }
+        }
+        // A lane whose particle is lost stops after that turn: every later
+        // update would only add NaN to windows that are still open (fixed
+        // below).
+        if (!alive) {
+            ++k;
+            break;
+        }
     }
 
-    // ---- windows a stopped warp would still have touched become NaN --------
+    // ---- windows a stopped lane would still have touched become NaN --------
     if (k < a.n_turns) {
         const double nan = dev::quiet_nan();
         const uint64_t left = a.n_turns - k;  // turns skipped
@@ -345,19 +389,16 @@ __global__ void __launch_bounds__(128, SPLIT ? 4 : 1) indicators_kernel(const Fu
                     ly_b[w * T + tid] = nan;
                 }
         }
-        if (do_t) {
+        if (DO_T) {
             const uint64_t first = a.tu_idx + k, last = a.tu_idx + k + left - 1;
             for (int w = 0; w < a.n_tu; ++w) {
                 const uint64_t len = tab_tu[w].len;
-                if (first < len) {
-                    t1x[w * T + tid] = nan;
-                    t1y[w * T + tid] = nan;
-                }
                 // window 2 is [len, 2 len): touched if it meets [first, last]
-                if (first < 2 * len && last >= len) {
-                    t2x[w * T + tid] = nan;
-                    t2y[w * T + tid] = nan;
-                }
+                const bool one = first < len, two = first < 2 * len && last >= len;
+                if (do_tx && one) t1x[w * T + tid] = nan;
+                if (do_ty && one) t1y[w * T + tid] = nan;
+                if (do_tx && two) t2x[w * T + tid] = nan;
+                if (do_ty && two) t2y[w * T + tid] = nan;
             }
         }
     }
@@ -391,22 +432,25 @@ __global__ void __launch_bounds__(128, SPLIT ? 4 : 1) indicators_kernel(const Fu
             a.ly_b[g] = ly_b[w * T + tid];
         }
     }
-    if (do_t) {
-        a.store_x[i] = store_x;
-        a.store_y[i] = store_y;
+    if (do_tx) a.store_x[i] = store_x;
+    if (do_ty) a.store_y[i] = store_y;
+    if (DO_T)
         for (int w = 0; w < a.n_tu; ++w) {
             const size_t g = size_t(tab_tu[w].orig) * n + i;
-            a.t1x[g] = t1x[w * T + tid];
-            a.t1y[g] = t1y[w * T + tid];
-            a.t2x[g] = t2x[w * T + tid];
-            a.t2y[g] = t2y[w * T + tid];
+            if (do_tx) {
+                a.t1x[g] = t1x[w * T + tid];
+                a.t2x[g] = t2x[w * T + tid];
+            }
+            if (do_ty) {
+                a.t1y[g] = t1y[w * T + tid];
+                a.t2y[g] = t2y[w * T + tid];
+            }
         }
-    }
 }
 
 // The matrix and the vector/tune work are split over two warps per particle
 // when both are requested (64 particles per block of 128 threads).
-template <bool OCT, bool DO_M, bool DO_V, bool DO_T>
+template <bool OCT, bool DO_M, bool DO_V, bool DO_T, bool PLANES = false>
 cudaError_t launch4(const FusedArgs &a, cudaStream_t s) {
     constexpr int threads = 128;
     constexpr bool split = DO_M && (DO_V || DO_T);
@@ -414,7 +458,7 @@ cudaError_t launch4(const FusedArgs &a, cudaStream_t s) {
     const size_t slots = size_t(a.n_mb) + 2 * size_t(a.n_ly) + 4 * size_t(a.n_tu);
     const size_t tables = (size_t(a.n_mb) + a.n_ly + a.n_tu) * sizeof(WinEntry);
     const size_t smem = slots * per_block * sizeof(double) + tables;
-    auto k = indicators_kernel<OCT, DO_M, DO_V, DO_T, split>;
+    auto k = indicators_kernel<OCT, DO_M, DO_V, DO_T, split, false, PLANES>;
     if (smem > 48 * 1024) {
         const cudaError_t e =
             cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
@@ -425,10 +469,16 @@ cudaError_t launch4(const FusedArgs &a, cudaStream_t s) {
     return cudaGetLastError();
 }
 
+// Lyapunov and tune windows open per turn from which the y plane's tunes are
+// better off with the matrix work: between the 5.6 and the 10.8 measured above.
+constexpr double kPlanesOpen = 8.0;
+
 template <bool OCT>
 cudaError_t launch_oct(const FusedArgs &a, cudaStream_t s) {
     const bool m = a.M != nullptr, v = a.V != nullptr, t = a.store_x != nullptr;
-    if (m && v && t) return launch4<OCT, true, true, true>(a, s);
+    if (m && v && t)
+        return a.open_windows > kPlanesOpen ? launch4<OCT, true, true, true, true>(a, s)
+                                            : launch4<OCT, true, true, true>(a, s);
     if (m && v) return launch4<OCT, true, true, false>(a, s);
     if (m && t) return launch4<OCT, true, false, true>(a, s);
     if (v && t) return launch4<OCT, false, true, true>(a, s);

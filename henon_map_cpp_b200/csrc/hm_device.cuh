@@ -640,6 +640,36 @@ __device__ __forceinline__ void jacobian_matvec4_exact(const double a[16], const
                      Rn::mul(a[15], v[3]));
 }
 
+// ---- division by a number whose reciprocal is at hand ---------------------------
+// RN(a / b) from y = RN(1 / b) by Markstein's correction (P. Markstein,
+// "Computation of elementary functions on the IBM RISC System/6000
+// processor", IBM J. Res. Dev. 34 (1990) 111-119): when q is within one unit
+// in the last place of a / b, RN(q + y RN(a - b q)) is a / b correctly
+// rounded, the residual being exact.  RN(a y) may be 1.5 units off, so it is
+// corrected twice.  Five FP64 instructions where a division is about 25 in
+// all, for the divisions of a turn that share a divisor.  The residuals must
+// not underflow and nothing may overflow: neither div_rare(a) nor
+// divisor_rare(b).
+__device__ __forceinline__ double div_by(double a, double b, double y) {
+    const double q0 = Rn::mul(a, y);
+    const double q1 = fma(fma(-b, q0, a), y, q0);
+    return fma(fma(-b, q1, a), y, q1);
+}
+
+// Dividends that div_by must not be given: zeros (the sign of the quotient),
+// |a| < 2^-800, |a| >= 2^800 and infinities.  A NaN may pass: the quotient
+// is NaN either way.
+__device__ __forceinline__ bool div_rare(double a) {
+    const uint32_t h = abs_hi(a);
+    return h < 0x0df00000u || (h >= 0x71f00000u && h <= 0x7ff00000u);
+}
+
+// Divisors likewise: all but 2^-100 <= |b| < 2^100 and NaN.
+__device__ __forceinline__ bool divisor_rare(double b) {
+    const uint32_t h = abs_hi(b);
+    return h < 0x39b00000u || (h >= 0x46300000u && h <= 0x7ff00000u);
+}
+
 // True when the double is neither infinite nor NaN (exponent field not all
 // ones), tested on the integer pipe.
 __device__ __forceinline__ bool finite_bits(double v) {

@@ -336,6 +336,8 @@ struct FusedArgs {
     double kick_module;
     unsigned long long kick_seed;
     int inverse;
+    // Lyapunov plus tune windows open per turn, averaged over the launch.
+    double open_windows;
 };
 
 cudaError_t launch_indicators(const FusedArgs &a, cudaStream_t s);

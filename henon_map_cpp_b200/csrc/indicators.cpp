@@ -698,6 +698,15 @@ hm_status track_indicators(hm_tracker *t, hm_particles *p, uint32_t n_turns, dou
         a.mb_idx = s.megno_birkhoff ? s.megno_birkhoff->idx : 0;
         a.ly_idx = s.lyapunov ? s.lyapunov->idx : 0;
         a.tu_idx = s.tune ? s.tune->idx : 0;
+        double open = 0.0;  // window-turns of this launch
+        auto count = [&](uint64_t limit, uint64_t idx) {
+            open += double(std::min<uint64_t>(limit > idx ? limit - idx : 0u, len));
+        };
+        if (s.lyapunov)
+            for (uint64_t w : s.lyapunov->w.len) count(w, s.lyapunov->idx);
+        if (s.tune)
+            for (uint64_t w : s.tune->w.len) count(2 * w, s.tune->idx);
+        a.open_windows = open / double(len);
         HM_CUDA_TRY(hm::launch_indicators(a, 0));
         HM_CUDA_TRY(cudaDeviceSynchronize());
         if (inverse) {
