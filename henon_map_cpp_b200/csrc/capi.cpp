@@ -552,14 +552,12 @@ hm_status compute_tables(hm_tracker *t, uint32_t n_turns, double omega_x, double
 
 namespace hm {
 
-// (Re)allocates the device arrays of p for p->n_total particles and uploads
-// coordinates, steps and the host-side bookkeeping vectors.
-hm_status particles_upload(hm_particles *p, const double *x, const double *px,
-                           const double *y, const double *py) {
+// (Re)allocates the device arrays of p for p->n_total particles; on failure
+// they are as before (the slab aside, which the caller may have taken).
+hm_status particles_alloc(hm_particles *p) {
     const size_t n = p->n_total;
     hm::DeviceBuffer *cur[4] = {&p->x, &p->px, &p->y, &p->py};
     hm::DeviceBuffer *ini[4] = {&p->x0d, &p->px0d, &p->y0d, &p->py0d};
-    const double *src[4] = {x, px, y, py};
     // One block for the thirteen arrays: an allocation waits for its stream
     // and a release for the device, 6-8 us each (150 us a set before).
     using hm::align256;
@@ -575,6 +573,18 @@ hm_status particles_upload(hm_particles *p, const double *x, const double *px,
     p->dghost.part_of(p->slab, n, &at);
     p->didx.part_of(p->slab, n * sizeof(uint64_t), &at);
     p->didx_base.part_of(p->slab, n * sizeof(uint64_t), &at);
+    return ok();
+}
+
+// Allocates the device arrays and uploads coordinates, steps and the
+// host-side bookkeeping vectors.
+hm_status particles_upload(hm_particles *p, const double *x, const double *px,
+                           const double *y, const double *py) {
+    const size_t n = p->n_total;
+    hm::DeviceBuffer *cur[4] = {&p->x, &p->px, &p->y, &p->py};
+    hm::DeviceBuffer *ini[4] = {&p->x0d, &p->px0d, &p->y0d, &p->py0d};
+    const double *src[4] = {x, px, y, py};
+    HM_TRY(particles_alloc(p));
     if (n == 0) return ok();
     const cudaStream_t s = 0;
     for (int f = 0; f < 4; ++f) {

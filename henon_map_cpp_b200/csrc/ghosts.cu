@@ -111,7 +111,7 @@ __global__ void __launch_bounds__(128) ghost_lyapunov_kernel(const GhostLyapunov
     }
     double lyap[G];
 #pragma unroll
-    for (int g = 0; g < G; ++g) lyap[g] = in_range ? a.lyap[size_t(g) * a.n_base + bb] : 0.0;
+    for (int g = 0; g < G; ++g) lyap[g] = in_range ? a.lyap[bb * G + g] : 0.0;
     const dev::Barrier bar = dev::make_barrier<ARITH>(a.b2bits);
     const double mu = a.mu, module = a.module;
     uint32_t turn = a.turn0;
@@ -185,7 +185,7 @@ __global__ void __launch_bounds__(128) ghost_lyapunov_kernel(const GhostLyapunov
         }
     }
 #pragma unroll
-    for (int g = 0; g < G; ++g) a.lyap[size_t(g) * a.n_base + b] = lyap[g];
+    for (int g = 0; g < G; ++g) a.lyap[b * G + g] = lyap[g];
 }
 
 template <int ARITH, bool OCT>
@@ -199,6 +199,31 @@ cudaError_t launch_ghosts_g(const GhostLyapunovArgs &a, cudaStream_t s) {
         default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();
+}
+
+// The arrays of a set with one more ghost per base particle, from those of
+// the set before (add_ghost, src/henon.cu:737-818): the entries there are, with
+// the state back at the initial conditions, then the ghosts, displaced by
+// `module` along one coordinate.
+__global__ void append_ghosts_kernel(const GhostArrays from, const GhostArrays to, size_t n,
+                                     size_t n_base, uint64_t ghost_index, int direction,
+                                     double module) {
+    const size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (i >= n + n_base) return;
+    const bool ghost = i >= n;
+    const size_t b = ghost ? i - n : i;  // base particles come first
+#pragma unroll
+    for (int f = 0; f < 4; ++f) {
+        double v = from.initial[f][b];
+        if (ghost && f == direction) v = Rn::add(v, module);
+        to.initial[f][i] = v;
+        to.current[f][i] = v;
+    }
+    to.steps[i] = 0u;
+    to.valid[i] = from.valid[b];
+    to.ghost[i] = ghost ? uint8_t(1) : from.ghost[b];
+    to.idx[i] = ghost ? ghost_index : from.idx[b];
+    to.idx_base[i] = ghost ? b : from.idx_base[b];
 }
 
 // idx = idx_base = i: the indices of a set without ghosts (particles_4d
@@ -216,6 +241,17 @@ __global__ void particle_indices_kernel(uint64_t *idx, uint64_t *idx_base, size_
 cudaError_t launch_particle_indices(uint64_t *idx, uint64_t *idx_base, size_t n, cudaStream_t s) {
     if (n == 0) return cudaSuccess;
     particle_indices_kernel<<<unsigned((n + 255) / 256), 256, 0, s>>>(idx, idx_base, n);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_append_ghosts(const GhostArrays &from, const GhostArrays &to, size_t n,
+                                 size_t n_base, uint64_t ghost_index, int direction,
+                                 double module, cudaStream_t s) {
+    const size_t total = n + n_base;
+    if (total == 0) return cudaSuccess;
+    append_ghosts_kernel<<<unsigned((total + 255) / 256), 256, 0, s>>>(from, to, n, n_base,
+                                                                       ghost_index, direction,
+                                                                       module);
     return cudaGetLastError();
 }
 

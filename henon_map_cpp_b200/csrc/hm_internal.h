@@ -547,6 +547,7 @@ cudaError_t launch_fft_peak(const double2 *buf, uint32_t len, size_t count, cons
 // at the given host coordinates, which become the initial conditions:
 // steps = 0 and valid = 1; ghost, idx and idx_base from the host mirrors
 // when they are built, else those of a set without ghosts (capi.cpp).
+hm_status particles_alloc(hm_particles *p);
 hm_status particles_upload(hm_particles *p, const double *x, const double *px, const double *y,
                            const double *py);
 // Builds p's host mirrors from the device copies, once (capi.cpp).
@@ -569,8 +570,20 @@ struct GhostLyapunovArgs {
     double mu;
     long long b2bits;
     double module;
-    double *lyap;  // [n_ghosts][n_base] running sums of log(d / module)
+    double *lyap;  // [n_base][n_ghosts] running sums of log(d / module)
 };
+// The arrays of a particle set: current and initial {x, px, y, py}, steps, ...
+struct GhostArrays {
+    double *current[4], *initial[4];
+    uint32_t *steps;
+    uint8_t *valid, *ghost;
+    uint64_t *idx, *idx_base;
+};
+// One more ghost per base particle (the first n_base of n entries), displaced
+// along coordinate `direction` (0..3).
+cudaError_t launch_append_ghosts(const GhostArrays &from, const GhostArrays &to, size_t n,
+                                 size_t n_base, uint64_t ghost_index, int direction,
+                                 double module, cudaStream_t s);
 cudaError_t launch_ghost_lyapunov(const GhostLyapunovArgs &a, int arith, cudaStream_t s);
 int ghost_lyapunov_max_ghosts();
 
