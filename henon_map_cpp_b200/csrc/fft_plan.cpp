@@ -1,7 +1,7 @@
 // Plans of the shared-memory FFT tunes (fft_tune_kernel, tunes.cu).
 //
 // A plan holds, for windows of L samples, the factorisation of the
-// transform length M into radices 5, 3, 8, 4 and 2, the twiddles
+// transform length M into radices 5, 3, 16, 8, 4 and 2, the twiddles
 // exp(-2 pi i t / M) as two tables whose product gives any t < M (64-step
 // coarse values and the 64 fine ones; both fit in shared memory), and
 // either the position of each X_k after the forward network (M = L) or,
@@ -30,17 +30,24 @@ namespace {
 using cld = std::complex<long double>;
 
 // Radices of M: fives and threes first (the early stages, whose spans are
-// long), then eights and a four or a two (the late stages, short spans,
-// which the shared-memory swizzle spreads over the banks); false when M has
+// long), then the power of two in as few stages as radix 16 allows, of about
+// equal radices (2^13 = 16 8 8 8), the larger first; false when M has
 // another prime factor.
 bool factor(uint32_t M, std::vector<uint8_t> *rad) {
     rad->clear();
     uint32_t m = M;
-    for (uint32_t r : {5u, 3u, 8u, 4u, 2u})
+    for (uint32_t r : {5u, 3u})
         while (m % r == 0) {
             rad->push_back(uint8_t(r));
             m /= r;
         }
+    int bits = 0;
+    for (; m % 2 == 0; m /= 2) ++bits;
+    for (int left = (bits + 3) / 4; left > 0; --left) {
+        const int b = (bits + left - 1) / left;
+        rad->push_back(uint8_t(1 << b));
+        bits -= b;
+    }
     return m == 1 && rad->size() <= size_t(kFftMaxStages);
 }
 
@@ -64,7 +71,7 @@ void network_forward(std::vector<cld> &x, const std::vector<uint8_t> &rad) {
         const uint32_t span = N / r;
         for (uint32_t b0 = 0; b0 < M; b0 += N)
             for (uint32_t j = 0; j < span; ++j) {
-                cld v[8], y[8];
+                cld v[16], y[16];
                 for (uint32_t q = 0; q < r; ++q) v[q] = x[b0 + j + q * span];
                 for (uint32_t k = 0; k < r; ++k) {
                     y[k] = 0;
@@ -86,7 +93,7 @@ std::vector<double2> to_double2(const std::vector<cld> &v) {
 
 struct PlanEntry {
     FftPlanDev dev;
-    DeviceBuffer coarse, fine, pos, chirp, bhat;
+    DeviceBuffer coarse, fine, pos, freq, chirp, bhat;
 };
 
 struct FftPlans {
@@ -125,7 +132,7 @@ hm_status build_plan(uint32_t L, PlanEntry *e, bool *supported) {
     d.L = L;
     d.M = M;
     d.bluestein = blue ? 1 : 0;
-    d.swizzle = M % 8 == 0 ? 1 : 0;
+    d.swizzle = M % 8 != 0 || rad.back() % 2 != 0 ? 0 : (rad.back() == 16 ? 4 : 3);
     d.n_stages = int(rad.size());
     uint32_t N = M, prod = 1;
     for (size_t s = 0; s < rad.size(); ++s) {
@@ -156,8 +163,12 @@ hm_status build_plan(uint32_t L, PlanEntry *e, bool *supported) {
             }
             pos[k] = p;
         }
+        std::vector<uint32_t> freq(M);
+        for (uint32_t k = 0; k < M; ++k) freq[pos[k]] = k;
         HM_TRY(upload(e->pos, pos));
+        HM_TRY(upload(e->freq, freq));
         d.pos = e->pos.as<uint32_t>();
+        d.freq = e->freq.as<uint32_t>();
     } else {
         std::vector<cld> c(L), b(M, cld(0));
         for (uint64_t n = 0; n < L; ++n) c[n] = cis((n * n) % (2ull * L), 2ull * L);
@@ -168,7 +179,11 @@ hm_status build_plan(uint32_t L, PlanEntry *e, bool *supported) {
         }
         network_forward(b, rad);
         HM_TRY(upload(e->chirp, to_double2(c)));
-        HM_TRY(upload(e->bhat, to_double2(b)));
+        const uint32_t r = rad.empty() ? 1u : rad.back();
+        std::vector<cld> bt(M);
+        for (uint32_t t = 0; t < M / r; ++t)
+            for (uint32_t q = 0; q < r; ++q) bt[q * (M / r) + t] = b[t * r + q];
+        HM_TRY(upload(e->bhat, to_double2(bt)));
         d.chirp = e->chirp.as<double2>();
         d.bhat = e->bhat.as<double2>();
     }

@@ -494,7 +494,9 @@ constexpr uint32_t kFftMaxLen = 12800;
 struct FftPlanDev {
     uint32_t L = 0, M = 0;
     int bluestein = 0;
-    int swizzle = 0;  // shared-memory slots XOR-swizzled (M a multiple of 8)
+    // Shared-memory slots XOR-swizzled by the bits from this one on: 4 where
+    // the last radix is 16, 3 for 8, 4 and 2, 0 (not) for 5 and 3.
+    int swizzle = 0;
     int n_stages = 0;
     uint8_t radix[kFftMaxStages] = {};
     uint32_t stage_len[kFftMaxStages] = {};   // span of the stage's butterflies
@@ -503,8 +505,11 @@ struct FftPlanDev {
     const double2 *tw_coarse = nullptr;  // exp(-2 pi i 64 u / M), u < n_coarse
     const double2 *tw_fine = nullptr;    // exp(-2 pi i v / M), v < 64
     const uint32_t *pos = nullptr;       // direct: where X_k lies after the network
+    const uint32_t *freq = nullptr;      // direct: the k of the X_k that lies there
     const double2 *chirp = nullptr;      // Bluestein: exp(-i pi n^2 / L), n < L
-    const double2 *bhat = nullptr;       // Bluestein: the network's output for b
+    // Bluestein: the network's output for b; value q of the last stage's
+    // butterfly t at q M / r + t (r the last radix), as its threads read it.
+    const double2 *bhat = nullptr;
 };
 // The plan of windows of L samples on the current device (built once, kept
 // until exit); *plan is null when L needs the library path.

@@ -606,28 +606,39 @@ __global__ void fft_peak_kernel(const double2 *buf, uint32_t len, size_t count,
 
 // ---- FFT tunes in shared memory --------------------------------------------------
 // One block per row (plane, particle) of one window: the samples are read
-// from the orbit (mean subtracted, Hann window applied) into shared memory,
-// transformed there, and the block writes the interpolated peak.  The
-// transform of length M is an in-place mixed-radix network of radices 2, 3,
-// 4, 5 and 8.  Forward, decimation in frequency: stage s splits each block of
+// from the orbit (mean subtracted, Hann window applied), transformed in
+// shared memory, and the block writes the interpolated peak.  The transform of
+// length M is an in-place mixed-radix network of radices 2, 3, 4, 5, 8 and
+// 16.  Forward, decimation in frequency: stage s splits each block of
 // N = r * span values (radix r) into r butterflies of stride `span`,
 //     y_k = sum_q x_q w_r^{qk},  stored times w_N^{jk} (j: offset in the span),
 // which takes natural order in and leaves X_k at a digit-reversed position
 // (FftPlanDev::pos).  The inverse network runs the stages backwards with
 // conjugate twiddles applied before each butterfly (decimation in time),
 // which takes that order back to natural order (times M).  A window whose
-// length has no prime factor above 5 is transformed directly (M = L): its
-// samples, conjugated, are loaded at the forward network's positions, and
-// the inverse network returns conj(X_k) in natural order.  Other lengths
-// take Bluestein's convolution (L. Bluestein, "A linear filtering approach to the
-// computation of the discrete Fourier transform", IEEE Trans. Audio
-// Electroacoust. 18 (1970) 451-455), which uses both networks:
+// length has no prime factor above 5 is transformed directly (M = L) by the
+// forward network, and its peak is found in the digit-reversed order.
+// Other lengths take Bluestein's convolution (L. Bluestein, "A linear
+// filtering approach to the computation of the discrete Fourier transform",
+// IEEE Trans. Audio Electroacoust. 18 (1970) 451-455), which uses both
+// networks:
 //     X_k = c_k sum_n (z_n c_n) conj(c_{k-n}),  c_n = exp(-i pi n^2 / L),
 // the cyclic convolution of length M >= 2L - 1 being the inverse network of
 // the pointwise product of the forward network's outputs (that of b_m =
 // conj(c_m) is precomputed, in the same order).  |c_k| = 1 and the peak
 // interpolation depends on magnitude ratios only, so the peak is taken on
 // |conv_k| directly.
+//
+// A row's time is its passes over shared memory with a barrier after each, so
+// there are as few as possible: radix 16 where the power of two allows; the
+// first stage takes its values from the orbit; Bluestein's last forward stage,
+// the product and the first inverse stage, which work on the same values,
+// are one pass; the last stage looks for the maximum as it writes.  2^13
+// values: 8 passes instead of 13.  32,768 rows, before -> now: windows of 1001
+// (M = 2048) 1.16 -> 1.03 ms, 4001 (8192) 6.67 -> 5.33, 5001 (10240) 7.91 ->
+// 6.6, 10,000 (direct) 6.1 -> 6.2; 38-41 % of the issue slots and 24-37 % of the
+// FP64 pipe busy: one row fills an SM, so its passes, arithmetic and reads
+// of the orbit follow one another.
 
 __device__ __forceinline__ double2 c_add(double2 a, double2 b) {
     return make_double2(a.x + b.x, a.y + b.y);
@@ -656,7 +667,7 @@ __device__ __forceinline__ double2 fft_twiddle(const double2 *coarse, const doub
     return c_mul(coarse[t >> 6], fine[t & 63u]);
 }
 
-// The DFT of R values in registers (R = 2, 3, 4, 5, 8), forward
+// The DFT of R values in registers (R = 2, 3, 4, 5, 8, 16), forward
 // (w = exp(-2 pi i / R)) or inverse (conjugate w).
 template <bool INV>
 __device__ __forceinline__ void dft4(double2 &x0, double2 &x1, double2 &x2, double2 &x3) {
@@ -669,9 +680,53 @@ __device__ __forceinline__ void dft4(double2 &x0, double2 &x1, double2 &x2, doub
     x3 = INV ? c_sub(t1, it3) : c_add(t1, it3);
 }
 
+// a w16^m, w16 = exp(-2 pi i / 16) (INV: the conjugate); m = 0..9 as needed.
+template <int M16, bool INV>
+__device__ __forceinline__ double2 mul_w16(double2 a) {
+    constexpr double h = 0.70710678118654752440;   // cos(pi / 4)
+    constexpr double c1 = 0.92387953251128675613;  // cos(pi / 8)
+    constexpr double s1 = 0.38268343236508977173;  // sin(pi / 8)
+    if constexpr (M16 == 0) return a;
+    if constexpr (M16 == 4) return INV ? c_i(a) : make_double2(a.y, -a.x);
+    if constexpr (M16 == 2)
+        return INV ? make_double2(h * (a.x - a.y), h * (a.x + a.y))
+                   : make_double2(h * (a.x + a.y), h * (a.y - a.x));
+    if constexpr (M16 == 6)
+        return INV ? make_double2(-h * (a.x + a.y), h * (a.x - a.y))
+                   : make_double2(h * (a.y - a.x), -h * (a.x + a.y));
+    // 1: (c1, -s1), 3: (s1, -c1), 9: (-c1, s1)
+    constexpr double re = M16 == 1 ? c1 : (M16 == 3 ? s1 : -c1);
+    constexpr double im = M16 == 1 ? -s1 : (M16 == 3 ? -c1 : s1);
+    return INV ? c_mulc(a, make_double2(re, im)) : c_mul(a, make_double2(re, im));
+}
+
 template <int R, bool INV>
 __device__ __forceinline__ void dft_small(double2 (&v)[R]) {
-    if constexpr (R == 2) {
+    if constexpr (R == 16) {
+        // X_{a + 4 b} = sum_c w16^{ca} w4^{cb} sum_d x_{4d + c} w4^{da}
+#pragma unroll
+        for (int c = 0; c < 4; ++c) dft4<INV>(v[c], v[4 + c], v[8 + c], v[12 + c]);
+        v[5] = mul_w16<1, INV>(v[5]);
+        v[6] = mul_w16<2, INV>(v[6]);
+        v[7] = mul_w16<3, INV>(v[7]);
+        v[9] = mul_w16<2, INV>(v[9]);
+        v[10] = mul_w16<4, INV>(v[10]);
+        v[11] = mul_w16<6, INV>(v[11]);
+        v[13] = mul_w16<3, INV>(v[13]);
+        v[14] = mul_w16<6, INV>(v[14]);
+        v[15] = mul_w16<9, INV>(v[15]);
+#pragma unroll
+        for (int a = 0; a < 4; ++a) dft4<INV>(v[4 * a], v[4 * a + 1], v[4 * a + 2], v[4 * a + 3]);
+        // v[4a + b] holds X_{a + 4b}
+#pragma unroll
+        for (int a = 0; a < 4; ++a)
+#pragma unroll
+            for (int b = a + 1; b < 4; ++b) {
+                const double2 t = v[4 * a + b];
+                v[4 * a + b] = v[4 * b + a];
+                v[4 * b + a] = t;
+            }
+    } else if constexpr (R == 2) {
         const double2 a = v[0], b = v[1];
         v[0] = c_add(a, b);
         v[1] = c_sub(a, b);
@@ -730,69 +785,74 @@ __device__ __forceinline__ void dft_small(double2 (&v)[R]) {
     }
 }
 
-// Shared-memory slot of row value i: with SWZ the low three bits of i (its
-// place among 8 consecutive values, one 128-byte bank row of double2) are
-// XORed with the next three, so that the small strides of the last stages
-// (radices 8, 4, 2 run last) fall into different banks.  A bijection on
-// every aligned group of 8, so rows of a multiple of 8 values stay in place.
-template <bool SWZ>
+// Shared-memory slot of row value i: with SWZ (3 or 4) the low three bits of
+// i (its place among 8 consecutive values, one 128-byte bank row of double2)
+// are XORed with the three from bit SWZ on, so that the small strides of the
+// last stages fall into different banks: a last stage of radix 16 has its
+// threads 16 values apart, one of radix 8, 4 or 2 at most 8.  A bijection
+// on every aligned group of 8, so rows of a multiple of 8 values stay in
+// place.
+template <int SWZ>
 __device__ __forceinline__ uint32_t slot(uint32_t i) {
-    return SWZ ? (i ^ ((i >> 3) & 7u)) : i;
+    return SWZ ? (i ^ ((i >> SWZ) & 7u)) : i;
 }
 
-// w^k for k < 8 from w, w^2 and w^4 (at most two products deep).
-__device__ __forceinline__ double2 twiddle_pow(int k, double2 w1, double2 w2, double2 w4) {
-    switch (k) {
-        case 1: return w1;
-        case 2: return w2;
-        case 3: return c_mul(w1, w2);
-        case 4: return w4;
-        case 5: return c_mul(w1, w4);
-        case 6: return c_mul(w2, w4);
-        default: return c_mul(c_mul(w1, w2), w4);
+// The twiddles w^k, k < R, w = exp(-2 pi i t / M): w, w^4 and w^8 from the
+// tables, the others at most three products from those.
+template <int R>
+__device__ __forceinline__ void twiddles(double2 (&w)[R], const double2 *tc, const double2 *tf,
+                                         uint32_t t) {
+    w[0] = make_double2(1.0, 0.0);
+    w[1] = fft_twiddle(tc, tf, t);
+    if constexpr (R > 2) w[2] = c_mul(w[1], w[1]);
+    if constexpr (R > 3) w[3] = c_mul(w[1], w[2]);
+    if constexpr (R > 4) w[4] = R > 5 ? fft_twiddle(tc, tf, 4u * t) : c_mul(w[2], w[2]);
+    if constexpr (R > 5) {
+#pragma unroll
+        for (int k = 5; k < 8; ++k) w[k] = c_mul(w[4], w[k - 4]);
+    }
+    if constexpr (R > 8) {
+        w[8] = fft_twiddle(tc, tf, 8u * t);
+#pragma unroll
+        for (int k = 9; k < 16; ++k) w[k] = c_mul(w[8], w[k - 8]);
     }
 }
 
-// One stage of radix R over row[0, M): butterfly b (b < M / R) covers
-// block b / span at offset j = b % span; the twiddles w_N^{jk}, N = R span,
-// are exp(-2 pi i j k prod / M) = w^k with w from the tables.  Forward:
-// butterfly, then twiddles; inverse: conjugate twiddles, then the inverse
-// butterfly.  A stage of span 1 has j = 0 and no twiddles (TW false).
-template <int R, bool INV, bool SWZ, bool TW>
-__device__ __forceinline__ void fft_stage(double2 *row, uint32_t M, uint32_t span, uint32_t prod,
-                                          const double2 *tc, const double2 *tf) {
-    const uint32_t nb = M / R, T = blockDim.x;
-    uint32_t blk = threadIdx.x / span, j = threadIdx.x - blk * span;
+// First maximum of |X_k|^2 (monotone in |X_k|), ties to the smallest k.
+struct Peak {
+    double m2;
+    uint32_t k;
+    __device__ __forceinline__ void see(double2 v, uint32_t at) {
+        const double m = v.x * v.x + v.y * v.y;
+        if (m > m2 || (m == m2 && at < k)) {
+            m2 = m;
+            k = at;
+        }
+    }
+};
+
+// A row, or a part of it that later stages keep to themselves: its plan, its
+// values, the twiddle tables in shared memory, and the threads that work on
+// it.
+struct FftRow {
+    const FftPlanDev &pl;
+    double2 *row;
+    const double2 *tc, *tf;
+    uint32_t off, size;  // the part's values
+    uint32_t t, T;       // this thread's index among the part's threads
+};
+
+// Butterflies t, t + T, ... of a stage of radix R: block b / span at offset
+// j = b % span, kept without divisions.
+template <int R, class F>
+__device__ __forceinline__ void butterflies(const FftRow &r, uint32_t span, F body) {
+    const uint32_t nb = r.size / R, T = r.T;
+    uint32_t blk = r.t / span, j = r.t - blk * span;
     const uint32_t dq = T / span, dr = T - dq * span;
-    constexpr int kUnroll = R >= 8 ? 1 : 2;  // radix 8 fills the registers alone
+    constexpr int kUnroll = R >= 8 ? 1 : 2;  // larger radices fill the registers alone
 #pragma unroll kUnroll
-    for (uint32_t b = threadIdx.x; b < nb; b += T) {
-        const uint32_t base = blk * span * R + j;
-        double2 w1 = make_double2(1.0, 0.0), w2 = w1, w4 = w1;
-        if (TW) {
-            w1 = fft_twiddle(tc, tf, j * prod);
-            w2 = c_mul(w1, w1);
-            w4 = c_mul(w2, w2);
-        }
-        double2 v[R];
-        if (!INV) {
-#pragma unroll
-            for (int q = 0; q < R; ++q) v[q] = row[slot<SWZ>(base + q * span)];
-            dft_small<R, false>(v);
-#pragma unroll
-            for (int k = 0; k < R; ++k)
-                row[slot<SWZ>(base + k * span)] =
-                    (TW && k > 0) ? c_mul(v[k], twiddle_pow(k, w1, w2, w4)) : v[k];
-        } else {
-#pragma unroll
-            for (int q = 0; q < R; ++q) {
-                const double2 x = row[slot<SWZ>(base + q * span)];
-                v[q] = (TW && q > 0) ? c_mulc(x, twiddle_pow(q, w1, w2, w4)) : x;
-            }
-            dft_small<R, true>(v);
-#pragma unroll
-            for (int k = 0; k < R; ++k) row[slot<SWZ>(base + k * span)] = v[k];
-        }
+    for (uint32_t b = r.t; b < nb; b += T) {
+        body(j, r.off + blk * span * R + j);
         blk += dq;
         j += dr;
         if (j >= span) {
@@ -802,36 +862,104 @@ __device__ __forceinline__ void fft_stage(double2 *row, uint32_t M, uint32_t spa
     }
 }
 
-template <int R, bool INV, bool SWZ>
-__device__ __forceinline__ void fft_stage_any(double2 *row, uint32_t M, uint32_t span,
-                                              uint32_t prod, const double2 *tc,
-                                              const double2 *tf) {
-    if (span == 1) fft_stage<R, INV, SWZ, false>(row, M, span, prod, tc, tf);
-    else fft_stage<R, INV, SWZ, true>(row, M, span, prod, tc, tf);
+// Where a stage's values come from and go to.
+enum : int {
+    kFromRow = 0,   // row to row
+    kFromOrbit = 1, // the first forward stage: value i is in(i)
+    kToPeak = 2,    // the last stage: also seen by the peak
+};
+
+// One stage of radix R: forward, butterfly then twiddles; inverse, conjugate
+// twiddles then the inverse butterfly.  A stage of span 1 has j = 0 and no
+// twiddles (TW false).  The twiddles w_N^{jk}, N = R span, are
+// exp(-2 pi i j k prod / M).
+template <int R, bool INV, int SWZ, bool TW, int MODE, class In>
+__device__ __forceinline__ void fft_stage(const FftRow &r, uint32_t span, uint32_t prod, In in,
+                                          Peak &peak) {
+    double2 *const row = r.row;
+    butterflies<R>(r, span, [&](uint32_t j, uint32_t base) {
+        double2 v[R], w[R];
+        if constexpr (TW) twiddles<R>(w, r.tc, r.tf, j * prod);
+#pragma unroll
+        for (int q = 0; q < R; ++q) {
+            if constexpr (MODE == kFromOrbit) v[q] = in(base + q * span);
+            else v[q] = row[slot<SWZ>(base + q * span)];
+            if constexpr (TW && INV)
+                if (q > 0) v[q] = c_mulc(v[q], w[q]);
+        }
+        dft_small<R, INV>(v);
+#pragma unroll
+        for (int k = 0; k < R; ++k) {
+            if constexpr (TW && !INV)
+                if (k > 0) v[k] = c_mul(v[k], w[k]);
+            const uint32_t at = base + k * span;
+            row[slot<SWZ>(at)] = v[k];
+            if constexpr (MODE == kToPeak) {
+                if constexpr (INV) {
+                    if (at < r.pl.L) peak.see(v[k], at);
+                } else {
+                    peak.see(v[k], r.pl.freq[at]);
+                }
+            }
+        }
+    });
 }
 
-// The forward (decimation in frequency) or inverse (decimation in time)
-// network in place over the row; the caller synchronises before.
-template <bool INV, bool SWZ>
-__device__ void fft_network(double2 *row, const FftPlanDev &pl, const double2 *tc,
-                            const double2 *tf) {
-    for (int t = 0; t < pl.n_stages; ++t) {
-        const int s = INV ? pl.n_stages - 1 - t : t;
-        const uint32_t span = pl.stage_len[s], prod = pl.stage_prod[s];
-        switch (pl.radix[s]) {
-            case 8: fft_stage_any<8, INV, SWZ>(row, pl.M, span, prod, tc, tf); break;
-            case 4: fft_stage_any<4, INV, SWZ>(row, pl.M, span, prod, tc, tf); break;
-            case 2: fft_stage_any<2, INV, SWZ>(row, pl.M, span, prod, tc, tf); break;
-            case 5: fft_stage_any<5, INV, SWZ>(row, pl.M, span, prod, tc, tf); break;
-            default: fft_stage_any<3, INV, SWZ>(row, pl.M, span, prod, tc, tf); break;
-        }
-        __syncthreads();
+template <int R, bool INV, int SWZ, int MODE, class In>
+__device__ __forceinline__ void fft_stage_any(const FftRow &r, uint32_t span, uint32_t prod,
+                                              In in, Peak &peak) {
+    if (span == 1) fft_stage<R, INV, SWZ, false, MODE>(r, span, prod, in, peak);
+    else fft_stage<R, INV, SWZ, true, MODE>(r, span, prod, in, peak);
+}
+
+template <bool INV, int SWZ, int MODE, class In>
+__device__ void fft_stage_of(const FftRow &r, int s, In in, Peak &peak) {
+    const uint32_t span = r.pl.stage_len[s], prod = r.pl.stage_prod[s];
+    switch (r.pl.radix[s]) {
+        case 16: fft_stage_any<16, INV, SWZ, MODE>(r, span, prod, in, peak); break;
+        case 8: fft_stage_any<8, INV, SWZ, MODE>(r, span, prod, in, peak); break;
+        case 4: fft_stage_any<4, INV, SWZ, MODE>(r, span, prod, in, peak); break;
+        case 2: fft_stage_any<2, INV, SWZ, MODE>(r, span, prod, in, peak); break;
+        case 5: fft_stage_any<5, INV, SWZ, MODE>(r, span, prod, in, peak); break;
+        default: fft_stage_any<3, INV, SWZ, MODE>(r, span, prod, in, peak); break;
     }
 }
 
-constexpr int kFftThreadsMax = 1024;
+// Bluestein's turning point: the last forward stage (span 1, no twiddles),
+// the product with the kernel's transform and the first inverse stage.
+template <int R, int SWZ>
+__device__ __forceinline__ void fft_turn(const FftRow &r) {
+    const uint32_t nb = r.pl.M / R, b1 = (r.off + r.size) / R;
+    for (uint32_t b = r.off / R + r.t; b < b1; b += r.T) {
+        double2 v[R];
+#pragma unroll
+        for (int q = 0; q < R; ++q) v[q] = r.row[slot<SWZ>(b * R + q)];
+        dft_small<R, false>(v);
+#pragma unroll
+        for (int q = 0; q < R; ++q) v[q] = c_mul(v[q], __ldg(r.pl.bhat + q * nb + b));
+        dft_small<R, true>(v);
+#pragma unroll
+        for (int q = 0; q < R; ++q) r.row[slot<SWZ>(b * R + q)] = v[q];
+    }
+}
 
-template <bool SWZ>
+template <int SWZ>
+__device__ void fft_turn_of(const FftRow &r) {
+    switch (r.pl.radix[r.pl.n_stages - 1]) {
+        case 16: fft_turn<16, SWZ>(r); break;
+        case 8: fft_turn<8, SWZ>(r); break;
+        case 4: fft_turn<4, SWZ>(r); break;
+        case 2: fft_turn<2, SWZ>(r); break;
+        case 5: fft_turn<5, SWZ>(r); break;
+        default: fft_turn<3, SWZ>(r); break;
+    }
+}
+
+// 512 threads of 128 registers: one radix-16 butterfly each for 8192 values.
+constexpr int kFftThreadsMax = 512;
+constexpr uint32_t kFftGroups = 4;
+
+template <int SWZ>
 __global__ void __launch_bounds__(kFftThreadsMax) fft_tune_kernel(const FftTuneArgs a) {
     extern __shared__ __align__(16) double2 fft_sm[];
     __shared__ double red_m[kFftThreadsMax / 32];
@@ -873,28 +1001,54 @@ __global__ void __launch_bounds__(kFftThreadsMax) fft_tune_kernel(const FftTuneA
     }
     for (uint32_t t = threadIdx.x; t < pl.n_coarse; t += blockDim.x) tc[t] = pl.tw_coarse[t];
     for (uint32_t t = threadIdx.x; t < 64u; t += blockDim.x) tf[t] = pl.tw_fine[t];
+    __syncthreads();
     const double *q = plane ? a.y : a.x, *p = plane ? a.py : a.px;
     const double mq = mean_of(a.means, a.n, i, 2 * plane, a.S);
     const double mp = mean_of(a.means, a.n, i, 2 * plane + 1, a.S);
-    // z_k = ((q - mean) + i (p - mean)) h_k.  Bluestein: z_k c_k in natural
-    // order (zeros up to M) for the forward network.  Direct: conj(z_k) at
-    // the forward network's position of k, so that the inverse network
-    // gives conj(X_k) in natural order (the magnitudes are those of X_k).
+    // z_k = ((q - mean) + i (p - mean)) h_k, for Bluestein times c_k and with
+    // zeros up to M.
     const size_t o0 = i * a.stride_i + size_t(a.from) * a.stride_s;
     int nan_seen = 0;
-#pragma unroll 4
-    for (uint32_t k = threadIdx.x; k < pl.M; k += blockDim.x) {
-        double2 v = make_double2(0.0, 0.0);
-        if (k < pl.L) {
-            const size_t o = o0 + size_t(k) * a.stride_s;
-            const double re = centred(q[o], a.means, mq), im = centred(p[o], a.means, mp);
-            nan_seen |= isnan(re) || isnan(im);
-            const double hk = a.hann[k];
-            v = make_double2(re * hk, im * hk);
-            if (pl.bluestein) v = c_mul(v, pl.chirp[k]);
-            else v.y = -v.y;
+    auto in = [&](uint32_t k) {
+        if (k >= pl.L) return make_double2(0.0, 0.0);
+        const size_t o = o0 + size_t(k) * a.stride_s;
+        const double re = centred(q[o], a.means, mq), im = centred(p[o], a.means, mp);
+        nan_seen |= isnan(re) || isnan(im);
+        const double hk = a.hann[k];
+        const double2 z = make_double2(re * hk, im * hk);
+        return pl.bluestein ? c_mul(z, __ldg(pl.chirp + k)) : z;
+    };
+    const FftRow whole{pl, row, tc, tf, 0u, pl.M, threadIdx.x, blockDim.x};
+    const int last = pl.n_stages - 1;
+    // After a first stage of radix r the row is r independent transforms.
+    // Where r is a multiple of kFftGroups (powers of two) and there is a stage
+    // in between, each group of the block's threads takes its share of them
+    // through the middle stages, waiting for its own threads only: the groups
+    // drift apart, so that one's shared-memory passes overlap another's
+    // arithmetic (8192 values, 32,768 rows: 5.38 instead of 5.62 ms).  Lengths
+    // with fives keep them first: with 16 first and groups, 10240 values took
+    // 7.27 ms instead of 6.49, their butterflies not dealing out evenly.
+    const bool split = last > 1 && pl.radix[0] % kFftGroups == 0;
+    const uint32_t groups = split ? kFftGroups : 1u;
+    const uint32_t per = blockDim.x / groups, group = threadIdx.x / per;
+    const FftRow part{pl,  row, tc, tf, group * (pl.M / groups), pl.M / groups,
+                      threadIdx.x - group * per, per};
+    static_assert(kFftGroups == 4u, "one named barrier per group below");
+    auto part_sync = [&]() {  // (barrier numbers as constants: five in all, not sixteen)
+        switch (group) {
+            case 0: asm volatile("bar.sync 1, %0;" ::"r"(per) : "memory"); break;
+            case 1: asm volatile("bar.sync 2, %0;" ::"r"(per) : "memory"); break;
+            case 2: asm volatile("bar.sync 3, %0;" ::"r"(per) : "memory"); break;
+            default: asm volatile("bar.sync 4, %0;" ::"r"(per) : "memory"); break;
         }
-        row[slot<SWZ>(pl.bluestein ? k : pl.pos[k])] = v;
+    };
+    Peak peak{-1.0, 0xffffffffu};
+    int s = 0;  // forward stages done
+    if (last > 0) {
+        fft_stage_of<false, SWZ, kFromOrbit>(whole, 0, in, peak);
+        s = 1;
+    } else {
+        for (uint32_t k = threadIdx.x; k < pl.M; k += blockDim.x) row[slot<SWZ>(k)] = in(k);
     }
     // Without first-NaN records the window's own samples decide
     // (fft_tune_vec's rule, scanning the window).
@@ -904,26 +1058,32 @@ __global__ void __launch_bounds__(kFftThreadsMax) fft_tune_kernel(const FftTuneA
                 a.out[i * a.cols + 2 * size_t(a.out_cols[c]) + plane] = dev::quiet_nan();
         return;
     }
+    for (; s < last; ++s) {
+        fft_stage_of<false, SWZ, kFromRow>(part, s, in, peak);
+        part_sync();
+    }
     if (pl.bluestein) {
-        fft_network<false, SWZ>(row, pl, tc, tf);
-        for (uint32_t k = threadIdx.x; k < pl.M; k += blockDim.x)
-            row[slot<SWZ>(k)] = c_mul(row[slot<SWZ>(k)], pl.bhat[k]);
-        __syncthreads();
-    }
-    fft_network<true, SWZ>(row, pl, tc, tf);
-    auto at = [&](uint32_t k) { return row[slot<SWZ>(k)]; };
-    // First maximum of |X_k| (squared, monotone) over k < L; k grows within
-    // a thread, and ties across threads keep the smallest k.
-    double best = -1.0;
-    uint32_t best_k = 0xffffffffu;
-    for (uint32_t k = threadIdx.x; k < pl.L; k += blockDim.x) {
-        const double2 v = at(k);
-        const double m2 = v.x * v.x + v.y * v.y;
-        if (m2 > best) {
-            best = m2;
-            best_k = k;
+        fft_turn_of<SWZ>(part);
+        part_sync();
+        for (s = last - 1; s > 0; --s) {
+            fft_stage_of<true, SWZ, kFromRow>(part, s, in, peak);
+            part_sync();
         }
+        __syncthreads();
+        if (last > 0) {
+            fft_stage_of<true, SWZ, kToPeak>(whole, 0, in, peak);
+        } else {
+            for (uint32_t k = threadIdx.x; k < pl.L; k += blockDim.x) peak.see(row[slot<SWZ>(k)], k);
+        }
+    } else if (last >= 0) {
+        fft_stage_of<false, SWZ, kToPeak>(part, last, in, peak);
+    } else {  // one sample
+        if (threadIdx.x == 0) peak.see(row[0], 0u);
     }
+    // the peak's neighbours are read below, after the barrier of the reduction
+    auto at = [&](uint32_t k) { return row[slot<SWZ>(pl.bluestein || last < 0 ? k : pl.pos[k])]; };
+    double best = peak.m2;
+    uint32_t best_k = peak.k;
     const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     for (int o = 16; o > 0; o >>= 1) {
         const double ob = __shfl_down_sync(dev::kFullMask, best, o);
@@ -1058,19 +1218,19 @@ cudaError_t launch_fft_tunes(const FftTuneArgs &a, cudaStream_t s) {
     if (a.n == 0) return cudaSuccess;
     if (a.plan.M == 0 || a.plan.M > kFftMaxLen || a.plan.L == 0) return cudaErrorInvalidValue;
     const size_t smem = fft_tune_smem_bytes(a.plan);
-    auto kernel = a.plan.swizzle ? fft_tune_kernel<true> : fft_tune_kernel<false>;
+    auto kernel = a.plan.swizzle == 4   ? fft_tune_kernel<4>
+                  : a.plan.swizzle == 3 ? fft_tune_kernel<3>
+                                        : fft_tune_kernel<0>;
     if (smem > 40u * 1024u) {
         const cudaError_t e =
             cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
         if (e != cudaSuccess) return e;
     }
-    // About one radix-8 butterfly per thread and stage.  A row of 6144
-    // values or more fills most of an SM's shared memory, so its block takes
-    // up to 1024 threads; shorter rows take 256, so that several blocks share
-    // an SM.
-    const uint32_t want = (a.plan.M / 8u + 31u) / 32u * 32u;
-    const uint32_t cap = a.plan.M >= 6144u ? uint32_t(kFftThreadsMax) : 256u;
-    const int threads = int(std::min<uint32_t>(cap, std::max<uint32_t>(64u, want)));
+    // About one radix-16 butterfly per thread and stage, whole warps in each
+    // group.
+    const uint32_t step = 32u * kFftGroups;
+    const uint32_t want = (a.plan.M / 16u + step - 1u) / step * step;
+    const int threads = int(std::min<uint32_t>(kFftThreadsMax, std::max(step, want)));
     int dev = 0, sms = 0, per_sm = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);

@@ -394,3 +394,23 @@ def test_orbit_groups_and_segments(gpu, n, n_turns):
     for k in range(4):
         assert_bitwise(got[k], ref[k], f"coordinate {k}")
     np.testing.assert_array_equal(got[4], ref[4])
+
+
+def test_fft_tunes_of_every_radix(gpu):
+    # Radix 16 and what is left of a power of two, alone, behind fives and
+    # threes and in Bluestein's lengths; powers of two, whose middle stages
+    # run in groups of threads; transforms of one and two stages.
+    x, px, y, py = grid(0.25, 3, px0=0.001)
+    lengths = [5, 8, 9, 13, 17, 31, 32, 33, 80, 128, 255, 256, 257, 512, 1024, 2000, 2047, 2048,
+               4095, 4096, 5120, 6125, 8192, 10240, 12288]
+    n_turns = 12400
+    frm = [(29 * j) % 100 for j in range(len(lengths))]
+    to = [f + n - 1 for f, n in zip(frm, lengths)]
+    tr = C.Tracker(n_turns, *TUNES, "sps", NAN, 8.0, 0)
+    p = C.Particles(x, px, y, py)
+    _, f = C.tracker_orbit_tunes(tr, p, n_turns, 0.0, 10.0, frm, to, False, True)
+    orb = T.orbit(x, px, y, py, O.tables(n_turns, *TUNES, "sps", epsilon=8.0), n_turns, 0.0)
+    want = np.array([T.tune_vec(*(orb[c, :, i] for c in range(4)), frm, to, "fft")
+                     for i in range(x.size)])
+    assert np.isfinite(want).all()
+    _close(f, want, 1e-10, "fft")
