@@ -327,6 +327,8 @@ cudaError_t launch_batch_chunk(const BatchDev &b, int blocks, cudaStream_t s) {
     return cudaGetLastError();
 }
 
+int batch_chunk_warps() { return kWarps; }
+
 int batch_chunk_blocks_per_sm(int arith, int per_thread) {
     int n = 0;
     cudaError_t e;

@@ -388,6 +388,7 @@ cudaError_t launch_batch_plan(const BatchDev &b, uint32_t done_len, uint32_t nex
                               cudaStream_t s);
 cudaError_t launch_batch_chunk(const BatchDev &b, int blocks, cudaStream_t s);
 int batch_chunk_blocks_per_sm(int arith, int per_thread);
+int batch_chunk_warps();  // warps of a block of the chunk kernel
 
 // ---- adjoint (adjoint.cu / adjoint.cpp) ---------------------------------------
 
