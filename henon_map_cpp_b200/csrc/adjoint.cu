@@ -199,8 +199,8 @@ __global__ void __launch_bounds__(128) adjoint_kernel(const AdjointArgs a) {
 // errors of the reconstruction can grow only across one segment, and the
 // per-turn memory traffic of the replay variant disappears.
 // P particles per thread (particle index blockIdx.x * P * kThreads +
-// j * kThreads + threadIdx.x): P independent chains per thread hide the
-// latency of each turn's dependent FP64 operations.
+// j * kThreads + threadIdx.x): P independent chains that share each turn's
+// record (adjoint_per_thread chooses P).
 template <int ARITH, bool OCT, int P>
 __global__ void __launch_bounds__(kThreads) adjoint_inverse_kernel(const AdjointArgs a) {
     __shared__ __align__(16) double recs[2][kStage * kRec];
@@ -571,10 +571,22 @@ __global__ void __launch_bounds__(128) forward_loss_kernel(const AdjointArgs a) 
     }
 }
 
-// Particles per thread of the inverse-sweep kernel (1 or 2; results do not
-// depend on it).  Two chains per thread hide more of each turn's FP64
-// latency: 4.92 ms against 5.20 ms on 65,536 particles x 1e4 turns.
+// Most particles per thread of the inverse-sweep kernel (1 or 2; results do
+// not depend on it).
 int g_adjoint_per_thread = 2;
+
+// Particles per thread for n points.  Blocks of one particle per thread put
+// a warp on each scheduler, so an SM with w of them has w chains per
+// scheduler either way.  With w even, w / 2 warps of two chains cost a little
+// less than w warps of one (records read once for two, 2.5 to 4.5 % over w =
+// 2 .. 20).  With w odd, pairs would leave a scheduler w + 1 chains:
+// 3,000 turns at mu = 0.1 take 0.47 ms with one and 0.71 with two at w = 1
+// (18,644 points on 148 SMs), 1.05 and 1.32 at w = 3, 2.33 and 2.55 at w = 7.
+int adjoint_per_thread(size_t n) {
+    const size_t sms = size_t(sm_count());
+    const size_t w = ((n + kThreads - 1) / kThreads + sms - 1) / sms;
+    return g_adjoint_per_thread == 2 && w % 2 == 0 ? 2 : 1;
+}
 
 template <int ARITH>
 cudaError_t launch_a(const AdjointArgs &a, int mode, cudaStream_t s) {
@@ -584,7 +596,7 @@ cudaError_t launch_a(const AdjointArgs &a, int mode, cudaStream_t s) {
         if (oct) adjoint_kernel<ARITH, true><<<blocks, 128, 0, s>>>(a);
         else adjoint_kernel<ARITH, false><<<blocks, 128, 0, s>>>(a);
     } else if (mode == 3) {
-        if (g_adjoint_per_thread == 2) {
+        if (adjoint_per_thread(a.n) == 2) {
             const unsigned b = unsigned((a.n + 2 * kThreads - 1) / (2 * kThreads));
             if (oct) adjoint_inverse_kernel<ARITH, true, 2><<<b, kThreads, 0, s>>>(a);
             else adjoint_inverse_kernel<ARITH, false, 2><<<b, kThreads, 0, s>>>(a);

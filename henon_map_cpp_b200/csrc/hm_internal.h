@@ -16,6 +16,9 @@
 
 namespace hm {
 
+// Multiprocessors of the current device (cached per device ordinal; track.cu).
+int sm_count();
+
 // ---- error plumbing -------------------------------------------------------
 
 // Records `msg` as the calling thread's last error and returns `code`.
@@ -414,7 +417,7 @@ struct AdjointArgs {
 // mode 0: loss + reverse-mode gradients; 1: loss + forward-mode initial-
 // condition gradient (tangent map); 2: loss only.
 cudaError_t launch_adjoint(const AdjointArgs &a, int mode, cudaStream_t s);
-// Particles per thread of the inverse-sweep adjoint kernel (1 or 2).
+// Most particles per thread of the inverse-sweep adjoint kernel (1 or 2).
 void set_adjoint_per_thread(int p);
 int get_adjoint_per_thread();
 

@@ -301,15 +301,6 @@ __global__ void tune_add_kernel(const double *x, const double *px, const double 
     }
 }
 
-// Multiprocessors of the current device.
-int sm_count() {
-    int dev = 0, v = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || v <= 0)
-        return 1;
-    return v;
-}
-
 // Block of a kernel with windows: up to kThreads threads, the rows past the
 // first dealing with further windows while the set is small (a large one
 // keeps the device busy with one thread per particle, which then computes

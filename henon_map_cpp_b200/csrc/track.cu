@@ -22,6 +22,22 @@
 #include "hm_internal.h"
 
 namespace hm {
+
+// Multiprocessors of the current device (cached per device ordinal).
+int sm_count() {
+    constexpr int kMaxDevices = 64;
+    static std::atomic<int> cache[kMaxDevices];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return 1;
+    int v = cache[dev].load(std::memory_order_relaxed);
+    if (v <= 0) {
+        if (cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || v <= 0)
+            return 1;
+        cache[dev].store(v, std::memory_order_relaxed);
+    }
+    return v;
+}
+
 namespace {
 
 using dev::Barrier;
@@ -577,21 +593,6 @@ cudaError_t launch_s(const TrackChunk &c, unsigned blocks, int threads, cudaStre
         kernel<<<blocks, threads, smem, s>>>(c);
     }
     return cudaGetLastError();
-}
-
-// Multiprocessors of the current device (cached per device ordinal).
-int sm_count() {
-    constexpr int kMaxDevices = 64;
-    static std::atomic<int> cache[kMaxDevices];
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return 1;
-    int v = cache[dev].load(std::memory_order_relaxed);
-    if (v <= 0) {
-        if (cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || v <= 0)
-            return 1;
-        cache[dev].store(v, std::memory_order_relaxed);
-    }
-    return v;
 }
 
 constexpr uint64_t kMinBlocksPerSm = 2u;
