@@ -31,11 +31,10 @@ using dev::Particle;
 
 // Each warp of the persistent chunk kernel works on tiles of different
 // sets, so every warp stages its own set's turn records through shared
-// memory: while the warp runs the kStageTurns turns of one stage, each lane
-// holds kPerLane doubles of the next stage in registers (one coalesced
-// 256-byte load per kPerLane), and stores them into the warp's other buffer
-// at the end of the stage.  Without it, a warp whose set has few particles
-// left waits on an L2 round trip every few turns.
+// memory: while the warp runs the kStageTurns turns of one stage, the next
+// stage's records are copied asynchronously into the warp's other buffer.
+// Without it, a warp whose set has few particles left waits on an L2 round
+// trip every few turns.
 constexpr uint32_t kStageTurns = 32u;
 constexpr int kThreads = 128;
 constexpr int kWarps = kThreads / 32;

@@ -5,8 +5,10 @@
 // instruction-level parallelism).  The per-turn rotation record
 // {sin wx, cos wx, sin wy, cos wy} is the same for every live particle (all
 // live particles share the same `steps`), so each warp reads one broadcast
-// record per turn.  Losses are detected per turn; a lost particle is written
-// out at once (NaN coordinates, frozen steps) and survivors are re-compacted
+// record per turn.  Losses are looked for once per block of turns, and the
+// turn of a loss is found by redoing its block (dev::block_turns); a lost
+// particle is written out (NaN coordinates, frozen steps) and survivors are
+// re-compacted
 // into a dense list at the end of the chunk so that the next chunk's warps
 // are full.
 //

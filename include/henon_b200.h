@@ -109,8 +109,9 @@ hm_status hm_get_track_config(int *threads, int *per_thread,
  * warp and turn); otherwise one thread per block brings stage_turns turns
  * of records at a time into shared memory with a bulk copy (TMA,
  * double-buffered, bounded waits) and every warp reads them from there.
- * stage_turns is 0 or a power of two in [16, 512] (default 256); runs of
- * one chunk use direct reads.  Process-wide; results do not depend on it.
+ * stage_turns is 0 or a power of two in [16, 512] (default 512); a run of
+ * less than 16 turns uses direct reads.  Process-wide; results do not
+ * depend on it.
  * A staged copy that does not land within its bounded wait makes the call
  * return HM_ERR_TIMEOUT.  After HM_ERR_TIMEOUT the particles' coordinates
  * and steps are unspecified (the chunk that gave up may have moved some of
