@@ -49,6 +49,8 @@ constexpr int kPerThread = int(kStage) * kRec / kThreads;
 static_assert(kPerThread * kThreads == int(kStage) * kRec, "stage must split evenly");
 
 // Records of turns [lo, lo + kn) into registers, element e = 6 (turn - lo) + field.
+// Without GRAD there is no S_k (a.S may be null).
+template <bool GRAD>
 __device__ __forceinline__ void rec_load(double (&r)[kPerThread], const AdjointArgs &a,
                                          uint32_t lo, uint32_t kn) {
 #pragma unroll
@@ -58,7 +60,7 @@ __device__ __forceinline__ void rec_load(double (&r)[kPerThread], const AdjointA
         double v = 0.0;
         if (t < kn) {
             const size_t k = size_t(lo) + t;
-            v = f < 4u ? a.table[4u * k + f] : (f == 4u ? a.w[k] : a.S[k]);
+            v = f < 4u ? a.table[4u * k + f] : (f == 4u ? a.w[k] : (GRAD ? a.S[k] : 0.0));
         }
         r[q] = v;
     }
@@ -201,11 +203,19 @@ __global__ void __launch_bounds__(128) adjoint_kernel(const AdjointArgs a) {
 // P particles per thread (particle index blockIdx.x * P * kThreads +
 // j * kThreads + threadIdx.x): P independent chains that share each turn's
 // record (adjoint_per_thread chooses P).
-template <int ARITH, bool OCT, int P>
-__global__ void __launch_bounds__(kThreads) adjoint_inverse_kernel(const AdjointArgs a) {
+// Without GRAD it stops after the forward sweep and stores no checkpoint: the
+// loss alone: 1.78 ms for 65,536 points and 10^4 turns at mu = 0.1, 0.17 ms
+// for 18,644 points and 3,000 turns (3.21 and 0.90 ms with one thread per
+// point that loaded each turn's record and tested each turn).
+// Registers: enough for one chain's records loaded ahead (4 blocks per SM).
+// The compiler's own choice for P = 1 was 80 registers with spills, 0.47
+// instead of 0.425 ms for the gradients of 18,644 points and 3,000 turns;
+// with 9 chains per scheduler 2.97 and 3.00 ms.
+template <int ARITH, bool OCT, int P, bool GRAD>
+__global__ void __launch_bounds__(kThreads, P == 1 ? 4 : 3) adjoint_inverse_kernel(const AdjointArgs a) {
     __shared__ __align__(16) double recs[2][kStage * kRec];
     const size_t n = a.n;
-    const uint32_t N = a.n_turns, C = a.ckpt;
+    const uint32_t N = a.n_turns, C = GRAD ? a.ckpt : kStage;
     const uint32_t n_stages = (N + kStage - 1) / kStage;
     const dev::Barrier bar = dev::make_barrier<ARITH>(a.b2bits);
     size_t idx[P];
@@ -229,18 +239,19 @@ __global__ void __launch_bounds__(kThreads) adjoint_inverse_kernel(const Adjoint
 #pragma unroll
     for (int j = 0; j < P; ++j) {
         loss[j] = 0.0;
-        lost_at[j] = N;
+        // (the gradient call counts a point lost before the first turn as N)
+        lost_at[j] = GRAD || alive[j] ? N : 0u;
     }
     uint32_t next_ckpt = 0;  // turn of the next checkpoint store
     if (n_stages > 0) {
-        rec_load(next, a, 0u, min(kStage, N));
+        rec_load<GRAD>(next, a, 0u, min(kStage, N));
         rec_store(recs[0], next);
     }
     __syncthreads();
     for (uint32_t sg = 0; sg < n_stages; ++sg) {
         const uint32_t k0 = sg * kStage, kn = min(kStage, N - k0);
         const bool more = sg + 1 < n_stages;
-        if (more) rec_load(next, a, k0 + kStage, min(kStage, N - k0 - kStage));
+        if (more) rec_load<GRAD>(next, a, k0 + kStage, min(kStage, N - k0 - kStage));
         const double *R = recs[sg & 1u];
         // The stage's turns with no branch on their results (the tracking
         // kernel's scheme, track.cu turns_staged): the loss accumulates, and
@@ -269,7 +280,7 @@ __global__ void __launch_bounds__(kThreads) adjoint_inverse_kernel(const Adjoint
             if (k0 + kk == next_ckpt) {
 #pragma unroll
                 for (int j = 0; j < P; ++j)
-                    if (alive[j]) store4(a.ckpt_buf, (k0 + kk) / C, n, idx[j], coords(s[j]));
+                    if (GRAD && alive[j]) store4(a.ckpt_buf, (k0 + kk) / C, n, idx[j], coords(s[j]));
                 next_ckpt += C;
             }
             const uint32_t end = kk + min(kn - kk, next_ckpt - (k0 + kk));
@@ -298,7 +309,7 @@ __global__ void __launch_bounds__(kThreads) adjoint_inverse_kernel(const Adjoint
                 if (k == next_ckpt) {
 #pragma unroll
                     for (int j = 0; j < P; ++j)
-                        if (alive[j]) store4(a.ckpt_buf, k / C, n, idx[j], coords(s[j]));
+                        if (GRAD && alive[j]) store4(a.ckpt_buf, k / C, n, idx[j], coords(s[j]));
                     next_ckpt += C;
                 }
                 const double *rr = R + kRec * kk;
@@ -331,6 +342,7 @@ __global__ void __launch_bounds__(kThreads) adjoint_inverse_kernel(const Adjoint
             a.loss[idx[j]] = alive[j] ? loss[j] : 0.0;
             a.survived[idx[j]] = alive[j] ? 1 : 0;
         }
+    if (!GRAD) return;
 
     // ---- reverse sweep: turns N-1 .. 0 --------------------------------------------
     // The sweep carries half the adjoint (lambda / 2, with w_k in place of
@@ -359,7 +371,7 @@ __global__ void __launch_bounds__(kThreads) adjoint_inverse_kernel(const Adjoint
     // starts from its stored end state, the checkpoint after it.
     uint32_t seg_left = N - (n_seg ? n_seg - 1u : 0u) * C;
     if (__syncthreads_or(any_alive) && n_stages > 0) {
-        rec_load(next, a, N - min(kStage, N), min(kStage, N));
+        rec_load<GRAD>(next, a, N - min(kStage, N), min(kStage, N));
         rec_store(recs[0], next);
         __syncthreads();
         for (uint32_t sg = 0; sg < n_stages; ++sg) {
@@ -367,7 +379,7 @@ __global__ void __launch_bounds__(kThreads) adjoint_inverse_kernel(const Adjoint
             const bool more = sg + 1 < n_stages;
             if (more) {
                 const uint32_t kn2 = min(kStage, N - k0 - kStage);
-                rec_load(next, a, N - k0 - kStage - kn2, kn2);
+                rec_load<GRAD>(next, a, N - k0 - kStage - kn2, kn2);
             }
             // records of the table span [N - k0 - kn, N - k0), ascending
             const double *R = recs[sg & 1u];
@@ -461,7 +473,7 @@ __global__ void __launch_bounds__(kThreads) adjoint_inverse_kernel(const Adjoint
     }
 }
 
-// Forward mode: loss and, with TANGENT, g = sum_k w_k M_{k+1}^T grad A(x_{k+1})
+// Forward mode: loss and g = sum_k w_k M_{k+1}^T grad A(x_{k+1})
 // with M_{k+1} = DF_k ... DF_0 (DF_k = tangent_matrix at x_k, table[k]).
 // When a.g_th is given it also carries P_{k+1} = d x_{k+1} / d theta
 // (4 x 4: state by theta = (omega_x0, omega_y0, epsilon, mu)),
@@ -473,12 +485,12 @@ __global__ void __launch_bounds__(kThreads) adjoint_inverse_kernel(const Adjoint
 // turn's entry point, rotated with the turn.  Then
 //     dL/dtheta_j = sum_k w_k grad A(x_{k+1}) . P_{k+1}[:, j],
 // an independent check of the reverse sweep's theta gradient.
-template <int ARITH, bool OCT, bool TANGENT>
-__global__ void __launch_bounds__(128) forward_loss_kernel(const AdjointArgs a) {
+template <int ARITH, bool OCT>
+__global__ void __launch_bounds__(128) forward_tangent_kernel(const AdjointArgs a) {
     const size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= a.n) return;
     const size_t n = a.n;
-    const bool theta = TANGENT && a.g_th != nullptr;
+    const bool theta = a.g_th != nullptr;
     dev::Particle s = dev::make_particle(a.x0[i], a.px0[i], a.y0[i], a.py0[i]);
     const dev::Barrier bar = dev::make_barrier<ARITH>(a.b2bits);
     bool alive = !dev::is_lost(s.x, s.px, s.y, s.py);
@@ -492,12 +504,10 @@ __global__ void __launch_bounds__(128) forward_loss_kernel(const AdjointArgs a) 
         const dev::Turn t = dev::load_turn(a.table, k);
         double df[16];
         double u = 0.0, v = 0.0;
-        if (TANGENT) {
-            dev::tangent_matrix_exact(s.x, s.y, t, a.mu, df);
-            if (theta) {
-                u = s.x * fma(-3.0, s.yy, s.xx);  // x^3 - 3 x y^2
-                v = s.y * fma(-3.0, s.xx, s.yy);  // y^3 - 3 x^2 y
-            }
+        dev::tangent_matrix_exact(s.x, s.y, t, a.mu, df);
+        if (theta) {
+            u = s.x * fma(-3.0, s.yy, s.xx);  // x^3 - 3 x y^2
+            v = s.y * fma(-3.0, s.xx, s.yy);  // y^3 - 3 x^2 y
         }
         bool in;
         const double r = fwd<ARITH, OCT>(s, t, a.mu, bar, in);
@@ -506,68 +516,64 @@ __global__ void __launch_bounds__(128) forward_loss_kernel(const AdjointArgs a) 
             break;
         }
         loss = fma(a.w[k], r, loss);
-        if (TANGENT) {
-            double out[16];
+        double out[16];
+#pragma unroll
+        for (int rr = 0; rr < 4; ++rr)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                double acc = 0.0;
+#pragma unroll
+                for (int q = 0; q < 4; ++q) acc = fma(df[rr * 4 + q], M[q * 4 + c], acc);
+                out[rr * 4 + c] = acc;
+            }
+#pragma unroll
+        for (int q = 0; q < 16; ++q) M[q] = out[q];
+        const double w2 = 2.0 * a.w[k];
+        const double vv[4] = {w2 * s.x, w2 * s.px, w2 * s.y, w2 * s.py};
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+            g[c] = fma(M[c], vv[0], fma(M[4 + c], vv[1], fma(M[8 + c], vv[2], fma(M[12 + c], vv[3], g[c]))));
+        if (theta) {
 #pragma unroll
             for (int rr = 0; rr < 4; ++rr)
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
                     double acc = 0.0;
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) acc = fma(df[rr * 4 + q], M[q * 4 + c], acc);
+                    for (int q = 0; q < 4; ++q) acc = fma(df[rr * 4 + q], P[q * 4 + c], acc);
                     out[rr * 4 + c] = acc;
                 }
+            const double Sk = a.S[k];
+            const double f0 = fma(a.epsilon, Sk, 1.0);  // d omega(k) / d omega0
+            const double ex = a.omega_x0 * Sk, ey = a.omega_y0 * Sk;  // d omega / d eps
+            // columns: 0 omega_x0, 1 omega_y0, 2 epsilon, 3 mu
+            out[0 * 4 + 0] = fma(s.px, f0, out[0 * 4 + 0]);
+            out[1 * 4 + 0] = fma(-s.x, f0, out[1 * 4 + 0]);
+            out[2 * 4 + 1] = fma(s.py, f0, out[2 * 4 + 1]);
+            out[3 * 4 + 1] = fma(-s.y, f0, out[3 * 4 + 1]);
+            out[0 * 4 + 2] = fma(s.px, ex, out[0 * 4 + 2]);
+            out[1 * 4 + 2] = fma(-s.x, ex, out[1 * 4 + 2]);
+            out[2 * 4 + 2] = fma(s.py, ey, out[2 * 4 + 2]);
+            out[3 * 4 + 2] = fma(-s.y, ey, out[3 * 4 + 2]);
+            out[0 * 4 + 3] = fma(t.sx, u, out[0 * 4 + 3]);
+            out[1 * 4 + 3] = fma(t.cx, u, out[1 * 4 + 3]);
+            out[2 * 4 + 3] = fma(t.sy, v, out[2 * 4 + 3]);
+            out[3 * 4 + 3] = fma(t.cy, v, out[3 * 4 + 3]);
 #pragma unroll
-            for (int q = 0; q < 16; ++q) M[q] = out[q];
-            const double w2 = 2.0 * a.w[k];
-            const double vv[4] = {w2 * s.x, w2 * s.px, w2 * s.y, w2 * s.py};
+            for (int q = 0; q < 16; ++q) P[q] = out[q];
 #pragma unroll
             for (int c = 0; c < 4; ++c)
-                g[c] = fma(M[c], vv[0], fma(M[4 + c], vv[1], fma(M[8 + c], vv[2], fma(M[12 + c], vv[3], g[c]))));
-            if (theta) {
-#pragma unroll
-                for (int rr = 0; rr < 4; ++rr)
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) {
-                        double acc = 0.0;
-#pragma unroll
-                        for (int q = 0; q < 4; ++q) acc = fma(df[rr * 4 + q], P[q * 4 + c], acc);
-                        out[rr * 4 + c] = acc;
-                    }
-                const double Sk = a.S[k];
-                const double f0 = fma(a.epsilon, Sk, 1.0);  // d omega(k) / d omega0
-                const double ex = a.omega_x0 * Sk, ey = a.omega_y0 * Sk;  // d omega / d eps
-                // columns: 0 omega_x0, 1 omega_y0, 2 epsilon, 3 mu
-                out[0 * 4 + 0] = fma(s.px, f0, out[0 * 4 + 0]);
-                out[1 * 4 + 0] = fma(-s.x, f0, out[1 * 4 + 0]);
-                out[2 * 4 + 1] = fma(s.py, f0, out[2 * 4 + 1]);
-                out[3 * 4 + 1] = fma(-s.y, f0, out[3 * 4 + 1]);
-                out[0 * 4 + 2] = fma(s.px, ex, out[0 * 4 + 2]);
-                out[1 * 4 + 2] = fma(-s.x, ex, out[1 * 4 + 2]);
-                out[2 * 4 + 2] = fma(s.py, ey, out[2 * 4 + 2]);
-                out[3 * 4 + 2] = fma(-s.y, ey, out[3 * 4 + 2]);
-                out[0 * 4 + 3] = fma(t.sx, u, out[0 * 4 + 3]);
-                out[1 * 4 + 3] = fma(t.cx, u, out[1 * 4 + 3]);
-                out[2 * 4 + 3] = fma(t.sy, v, out[2 * 4 + 3]);
-                out[3 * 4 + 3] = fma(t.cy, v, out[3 * 4 + 3]);
-#pragma unroll
-                for (int q = 0; q < 16; ++q) P[q] = out[q];
-#pragma unroll
-                for (int c = 0; c < 4; ++c)
-                    gt[c] = fma(P[c], vv[0], fma(P[4 + c], vv[1], fma(P[8 + c], vv[2], fma(P[12 + c], vv[3], gt[c]))));
-            }
+                gt[c] = fma(P[c], vv[0], fma(P[4 + c], vv[1], fma(P[8 + c], vv[2], fma(P[12 + c], vv[3], gt[c]))));
         }
     }
     a.steps[i] = alive ? a.n_turns : k;
     a.survived[i] = alive ? 1 : 0;
     a.loss[i] = alive ? loss : 0.0;
-    if (TANGENT) {
 #pragma unroll
-        for (int c = 0; c < 4; ++c) a.g_ic[size_t(c) * n + i] = alive ? g[c] : 0.0;
-        if (theta) {
+    for (int c = 0; c < 4; ++c) a.g_ic[size_t(c) * n + i] = alive ? g[c] : 0.0;
+    if (theta) {
 #pragma unroll
-            for (int c = 0; c < 4; ++c) a.g_th[size_t(c) * n + i] = alive ? gt[c] : 0.0;
-        }
+        for (int c = 0; c < 4; ++c) a.g_th[size_t(c) * n + i] = alive ? gt[c] : 0.0;
     }
 }
 
@@ -578,14 +584,27 @@ int g_adjoint_per_thread = 2;
 // Particles per thread for n points.  Blocks of one particle per thread put
 // a warp on each scheduler, so an SM with w of them has w chains per
 // scheduler either way.  With w even, w / 2 warps of two chains cost a little
-// less than w warps of one (records read once for two, 2.5 to 4.5 % over w =
-// 2 .. 20).  With w odd, pairs would leave a scheduler w + 1 chains:
-// 3,000 turns at mu = 0.1 take 0.47 ms with one and 0.71 with two at w = 1
-// (18,644 points on 148 SMs), 1.05 and 1.32 at w = 3, 2.33 and 2.55 at w = 7.
+// less than w warps of one (records read once for two; up to 4 % over w = 2
+// .. 16, 1 % more only at w = 2 with mu = 0).  With w odd, pairs would leave a scheduler w + 1 chains:
+// 3,000 turns at mu = 0.1 take 0.43 ms with one and 0.71 with two at w = 1
+// (18,644 points on 148 SMs), 1.06 and 1.32 at w = 3, 2.35 and 2.55 at w = 7.
 int adjoint_per_thread(size_t n) {
     const size_t sms = size_t(sm_count());
     const size_t w = ((n + kThreads - 1) / kThreads + sms - 1) / sms;
     return g_adjoint_per_thread == 2 && w % 2 == 0 ? 2 : 1;
+}
+
+template <int ARITH, bool GRAD>
+void launch_inverse(const AdjointArgs &a, bool oct, int p, cudaStream_t s) {
+    const unsigned per_block = unsigned(p * kThreads);
+    const unsigned b = unsigned((a.n + per_block - 1) / per_block);
+    if (p == 2) {
+        if (oct) adjoint_inverse_kernel<ARITH, true, 2, GRAD><<<b, kThreads, 0, s>>>(a);
+        else adjoint_inverse_kernel<ARITH, false, 2, GRAD><<<b, kThreads, 0, s>>>(a);
+    } else {
+        if (oct) adjoint_inverse_kernel<ARITH, true, 1, GRAD><<<b, kThreads, 0, s>>>(a);
+        else adjoint_inverse_kernel<ARITH, false, 1, GRAD><<<b, kThreads, 0, s>>>(a);
+    }
 }
 
 template <int ARITH>
@@ -595,22 +614,13 @@ cudaError_t launch_a(const AdjointArgs &a, int mode, cudaStream_t s) {
     if (mode == 0) {
         if (oct) adjoint_kernel<ARITH, true><<<blocks, 128, 0, s>>>(a);
         else adjoint_kernel<ARITH, false><<<blocks, 128, 0, s>>>(a);
-    } else if (mode == 3) {
-        if (adjoint_per_thread(a.n) == 2) {
-            const unsigned b = unsigned((a.n + 2 * kThreads - 1) / (2 * kThreads));
-            if (oct) adjoint_inverse_kernel<ARITH, true, 2><<<b, kThreads, 0, s>>>(a);
-            else adjoint_inverse_kernel<ARITH, false, 2><<<b, kThreads, 0, s>>>(a);
-        } else {
-            const unsigned b = unsigned((a.n + kThreads - 1) / kThreads);
-            if (oct) adjoint_inverse_kernel<ARITH, true, 1><<<b, kThreads, 0, s>>>(a);
-            else adjoint_inverse_kernel<ARITH, false, 1><<<b, kThreads, 0, s>>>(a);
-        }
     } else if (mode == 1) {
-        if (oct) forward_loss_kernel<ARITH, true, true><<<blocks, 128, 0, s>>>(a);
-        else forward_loss_kernel<ARITH, false, true><<<blocks, 128, 0, s>>>(a);
-    } else {
-        if (oct) forward_loss_kernel<ARITH, true, false><<<blocks, 128, 0, s>>>(a);
-        else forward_loss_kernel<ARITH, false, false><<<blocks, 128, 0, s>>>(a);
+        if (oct) forward_tangent_kernel<ARITH, true><<<blocks, 128, 0, s>>>(a);
+        else forward_tangent_kernel<ARITH, false><<<blocks, 128, 0, s>>>(a);
+    } else {  // 3: gradients by the inverse sweep; 2: its forward sweep alone
+        const int p = adjoint_per_thread(a.n);
+        if (mode == 3) launch_inverse<ARITH, true>(a, oct, p, s);
+        else launch_inverse<ARITH, false>(a, oct, p, s);
     }
     return cudaGetLastError();
 }

@@ -51,3 +51,23 @@ def test_stretch_edges(gpu, n_turns, every, mu):
             continue
         rel = np.abs(x - y) / np.maximum(np.abs(y), 1e-300)
         assert np.median(rel) < tol, (k, np.median(rel))
+
+
+@pytest.mark.parametrize("n", [1, 300, 20_000])
+@pytest.mark.parametrize("n_turns", [1, 64, 129])
+@pytest.mark.parametrize("mu", [0.0, 0.1])
+def test_loss_alone(gpu, n, n_turns, mu):
+    """mode "loss" equals the tangent kernel's loss, loss turns and survival
+    bit for bit (one turn at a time there)."""
+    rng = np.random.default_rng(23)
+    pts = [torch.tensor(a, dtype=torch.float64, device="cuda")
+           for a in (rng.uniform(0, 0.6, n), rng.normal(0, 0.01, n),
+                     rng.uniform(0, 0.6, n), rng.normal(0, 0.01, n))]
+    if n > 1:
+        pts[2][n // 2] = math.nan
+    th = torch.tensor([2 * math.pi * TUNES[0], 2 * math.pi * TUNES[1], 16.0, mu],
+                      dtype=torch.float64)
+    a = AG.per_particle(*pts, th, n_turns, mode="loss")
+    b = AG.per_particle(*pts, th, n_turns, mode="tangent")
+    for k in ("loss", "steps", "survived"):
+        np.testing.assert_array_equal(a[k].cpu().numpy(), b[k].cpu().numpy(), err_msg=k)
