@@ -5,6 +5,7 @@
 #include <cstring>
 #include <mutex>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include <cuda_runtime.h>
@@ -224,7 +225,10 @@ hm_status DeviceBuffer::alloc(size_t nbytes) {
         HM_CUDA_TRY(cudaMemPoolTrimTo(pool, 0));
         got = cudaMallocFromPoolAsync(&p, nbytes, pool, 0);
     }
-    if (got != cudaSuccess) return cuda_fail(got, "cudaMallocFromPoolAsync");
+    if (got != cudaSuccess) {
+        cudaGetLastError();  // reported here, not by the next launch
+        return cuda_fail(got, "cudaMallocFromPoolAsync");
+    }
     // The block is ordered on the legacy stream; waiting for it makes it
     // usable from every stream, like a cudaMalloc block.
     const cudaError_t e = cudaStreamSynchronize(0);
@@ -552,17 +556,10 @@ hm_status compute_tables(hm_tracker *t, uint32_t n_turns, double omega_x, double
 
 namespace hm {
 
-// (Re)allocates the device arrays of p for p->n_total particles; on failure
-// they are as before (the slab aside, which the caller may have taken).
-hm_status particles_alloc(hm_particles *p) {
-    const size_t n = p->n_total;
+void particles_lay_out(hm_particles *p) {
+    const size_t n = p->slab.ptr ? p->n_total : 0;
     hm::DeviceBuffer *cur[4] = {&p->x, &p->px, &p->y, &p->py};
     hm::DeviceBuffer *ini[4] = {&p->x0d, &p->px0d, &p->y0d, &p->py0d};
-    // One block for the thirteen arrays: an allocation waits for its stream
-    // and a release for the device, 6-8 us each (150 us a set before).
-    using hm::align256;
-    HM_TRY(p->slab.alloc(8 * align256(n * sizeof(double)) + align256(n * sizeof(uint32_t)) +
-                         2 * align256(n) + 2 * align256(n * sizeof(uint64_t))));
     size_t at = 0;
     for (int f = 0; f < 4; ++f) {
         cur[f]->part_of(p->slab, n * sizeof(double), &at);
@@ -573,6 +570,20 @@ hm_status particles_alloc(hm_particles *p) {
     p->dghost.part_of(p->slab, n, &at);
     p->didx.part_of(p->slab, n * sizeof(uint64_t), &at);
     p->didx_base.part_of(p->slab, n * sizeof(uint64_t), &at);
+}
+
+// One block for the thirteen arrays: an allocation waits for its stream and a
+// release for the device, 6-8 us each (150 us a set before).
+static size_t slab_bytes(size_t n) {
+    return 8 * align256(n * sizeof(double)) + align256(n * sizeof(uint32_t)) + 2 * align256(n) +
+           2 * align256(n * sizeof(uint64_t));
+}
+
+hm_status particles_alloc(hm_particles *p) {
+    hm::DeviceBuffer fresh;
+    HM_TRY(fresh.alloc(slab_bytes(p->n_total)));
+    p->slab = std::move(fresh);
+    particles_lay_out(p);
     return ok();
 }
 

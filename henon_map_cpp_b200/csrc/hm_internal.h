@@ -552,11 +552,17 @@ cudaError_t launch_hann_gather(const double *q, const double *p, size_t n, uint3
 cudaError_t launch_fft_peak(const double2 *buf, uint32_t len, size_t count, const int *nan_flags,
                             double *out, size_t out_stride, size_t first, cudaStream_t s);
 
+// (Re)allocates the device arrays of p for p->n_total particles; on failure
+// they are as before (capi.cpp).
+hm_status particles_alloc(hm_particles *p);
+// Points the device arrays of p->n_total particles into p->slab (null without
+// one).
+void particles_lay_out(hm_particles *p);
 // (Re)allocates the device arrays of p's n_total particles and starts them
 // at the given host coordinates, which become the initial conditions:
 // steps = 0 and valid = 1; ghost, idx and idx_base from the host mirrors
-// when they are built, else those of a set without ghosts (capi.cpp).
-hm_status particles_alloc(hm_particles *p);
+// when they are built, else those of a set without ghosts.  Out of memory
+// leaves p's arrays as they were.
 hm_status particles_upload(hm_particles *p, const double *x, const double *px, const double *y,
                            const double *py);
 // Builds p's host mirrors from the device copies, once (capi.cpp).

@@ -94,23 +94,29 @@ hm::GhostArrays arrays_of(const hm_particles *p) {
     return a;
 }
 
-// add_ghost along a coordinate on the device.
+// add_ghost along a coordinate on the device; on failure p is as before
+// (without its tracking workspace).
 hm_status append_ghosts(hm_particles *p, double module, const std::string &dir) {
     const int direction = dir == "x" ? 0 : dir == "px" ? 1 : dir == "y" ? 2 : 3;
     const size_t n = p->n_total, nb = p->n_particles;
     const hm::GhostArrays from = arrays_of(p);
+    p->work.release();
     DeviceBuffer old = std::move(p->slab);
     p->n_total = n + nb;
-    const hm_status s = hm::particles_alloc(p);
+    hm_status s = hm::particles_alloc(p);
+    if (s == HM_OK) {
+        const cudaError_t e =
+            hm::launch_append_ghosts(from, arrays_of(p), n, nb, p->n_ghosts, direction, module, 0);
+        if (e != cudaSuccess) s = hm::cuda_fail(e, "append ghosts");
+    }
     if (s != HM_OK) {
         p->n_total = n;
         p->slab = std::move(old);
+        hm::particles_lay_out(p);
         return s;
     }
-    HM_CUDA_TRY(hm::launch_append_ghosts(from, arrays_of(p), n, nb, p->n_ghosts, direction, module, 0));
     p->n_ghosts += 1;
     p->live_step = 0;
-    p->work.release();
     return ok();  // releasing the old slab waits for the kernel
 }
 
@@ -131,9 +137,14 @@ hm_status hm_particles_add_ghost(hm_particles *p, double module, const char *dir
     // Directions along a coordinate need no host array: the new arrays are
     // written by one kernel from the ones there are (two ghosts of 65,536
     // particles 9 ms through the host mirrors).  Random directions draw from
-    // the host's generator, and a set that has host mirrors keeps them.
-    if (dir != "random" && !p->host_ready) return append_ghosts(p, module, dir);
+    // the host's generator, and a set that has host mirrors keeps them.  So
+    // does a set whose old and new arrays do not fit on the device together.
+    if (dir != "random" && !p->host_ready) {
+        const hm_status s = append_ghosts(p, module, dir);
+        if (s != HM_ERR_OOM) return s;
+    }
     HM_TRY(hm::particles_host_mirror(p));
+    const std::mt19937_64 rng = p->rng;
     const size_t n = p->n_total;
     std::vector<double> gx, gpx, gy, gpy;
     std::vector<uint8_t> gvalid;
@@ -163,10 +174,66 @@ hm_status hm_particles_add_ghost(hm_particles *p, double module, const char *dir
     p->idx.insert(p->idx.end(), gidx.begin(), gidx.end());
     p->idx_base.insert(p->idx_base.end(), gbase.begin(), gbase.end());
     p->n_total += gx.size();
-    p->n_ghosts += 1;
-    p->live_step = 0;
     p->work.release();
-    return hm::particles_upload(p, p->x0.data(), p->px0.data(), p->y0.data(), p->py0.data());
+    auto upload = [p] {
+        return hm::particles_upload(p, p->x0.data(), p->px0.data(), p->y0.data(), p->py0.data());
+    };
+    // The first m particles' state to (or, back, from) the host.
+    std::vector<double> state[4];
+    std::vector<uint32_t> steps;
+    auto copy_state = [&](size_t m, bool back) -> hm_status {
+        DeviceBuffer *cur[4] = {&p->x, &p->px, &p->y, &p->py};
+        steps.resize(m);
+        for (int f = 0; f < 4; ++f) {
+            state[f].resize(m);
+            HM_CUDA_TRY(back ? cudaMemcpy(cur[f]->ptr, state[f].data(), m * sizeof(double),
+                                          cudaMemcpyHostToDevice)
+                             : cudaMemcpy(state[f].data(), cur[f]->ptr, m * sizeof(double),
+                                          cudaMemcpyDeviceToHost));
+        }
+        HM_CUDA_TRY(back ? cudaMemcpy(p->steps.ptr, steps.data(), m * sizeof(uint32_t),
+                                      cudaMemcpyHostToDevice)
+                         : cudaMemcpy(steps.data(), p->steps.ptr, m * sizeof(uint32_t),
+                                      cudaMemcpyDeviceToHost));
+        return ok();
+    };
+    hm_status s = upload();
+    std::string why = hm_last_error();
+    bool given_up = false;
+    if (s == HM_ERR_OOM && n && copy_state(n, false) == HM_OK) {
+        // Once more in place of the old arrays.
+        given_up = true;
+        p->slab.release();
+        hm::particles_lay_out(p);
+        s = upload();
+        why = hm_last_error();
+    }
+    if (s == HM_OK) {
+        p->n_ghosts += 1;
+        p->live_step = 0;
+        return s;
+    }
+    // The set as before the call or, should its arrays no longer fit, empty.
+    auto cut = [p](size_t m) {
+        p->x0.resize(m);
+        p->px0.resize(m);
+        p->y0.resize(m);
+        p->py0.resize(m);
+        p->valid.resize(m);
+        p->ghost.resize(m);
+        p->idx.resize(m);
+        p->idx_base.resize(m);
+        p->n_total = m;
+    };
+    p->rng = rng;
+    cut(n);
+    if (given_up && (upload() != HM_OK || copy_state(n, true) != HM_OK)) {
+        p->slab.release();
+        cut(0);
+        p->n_particles = p->n_ghosts = 0;
+        hm::particles_lay_out(p);
+    }
+    return fail(s, why);
 }
 
 // renormalize (src/henon.cu:1257-1282): every ghost moved along its
