@@ -358,17 +358,24 @@ __global__ void __launch_bounds__(128, SPLIT ? 4 : 1) indicators_kernel(const Fu
             }
         }
         // A lane whose particle is lost stops after that turn: every later
-        // update would only add NaN to windows that are still open (fixed
-        // below).
+        // update would only make or add NaN (below).
         if (!alive) {
             ++k;
             break;
         }
     }
 
-    // ---- windows a stopped lane would still have touched become NaN --------
+    // ---- what a stopped lane would still have touched becomes NaN ----------
+    // Its own state (the first turn after the loss has a Jacobian and angles
+    // of NaN; with df_before, or in a warp that was lost before the first
+    // turn, that turn was not run), and the windows and samples still open.
     if (k < a.n_turns) {
         const double nan = dev::quiet_nan();
+#pragma unroll
+        for (int q = 0; q < 16; ++q) M[q] = nan;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) v[q] = nan;
+        m_l1 = m_l2 = m_l3 = b_l1 = store_x = store_y = nan;
         const uint64_t left = a.n_turns - k;  // turns skipped
         if (do_m && a.megno_l1)
             for (int j = 0; j < a.n_snap; ++j) {
