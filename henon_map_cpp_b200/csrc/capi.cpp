@@ -303,6 +303,10 @@ Workspace carve(void *base, size_t n) {
     return w;
 }
 
+// Particle-turns that the tracker enqueues before it waits for a count: half a
+// millisecond of exact turns at the full rate, 6 ms with kicks.
+constexpr uint64_t kMaxInFlight = uint64_t(1) << 29;
+
 }  // namespace
 
 // Advances n particles by n_turns turns of the map; *turns_done receives
@@ -373,6 +377,7 @@ hm_status track_driver(double *x, double *px, double *y, double *py,
     uint32_t done = 0;
     uint32_t chunk = cfg.chunk0;
     uint32_t n_in = uint32_t(n);
+    uint64_t in_flight = 0;  // particle-turns enqueued since the last wait
     int cur = -1;  // -1: the caller's arrays in identity order
     LaunchTimer timer;
     while (done < n_turns) {
@@ -414,14 +419,19 @@ hm_status track_driver(double *x, double *px, double *y, double *py,
         done += len;
         chunk = std::min<uint32_t>(chunk * 2u, cfg.chunk_max);
         if (last) break;
-        // The short chunks are enqueued without waiting for their survivor
-        // counts: the next grid covers the last count known, and its blocks
-        // past the list end at once.  A wait costs about 15 us, as much as
-        // 500 turns of a small set.
-        if (len < cfg.chunk_max && !timer.armed) {
+        // The short chunks of small sets are enqueued without waiting for
+        // their survivor counts: the next grid covers the last count known,
+        // and its blocks past the list end at once.  A wait costs about 15 us,
+        // as much as 500 turns of a small set.  The cancel callback is asked
+        // between all chunks; what is in flight when it is stays below about
+        // a millisecond of turns (ten with kicks).
+        in_flight += uint64_t(n_in) * len;
+        const bool wait = len >= cfg.chunk_max || in_flight >= kMaxInFlight || timer.armed;
+        if (!wait && !cancel_requested()) {
             cur = nxt;
             continue;
         }
+        in_flight = 0;
         uint32_t counters[3];  // count[0], count[1], fault
         HM_CUDA_TRY(cudaMemcpyAsync(counters, w.count[0], sizeof(counters),
                                     cudaMemcpyDeviceToHost, stream));
@@ -435,7 +445,7 @@ hm_status track_driver(double *x, double *px, double *y, double *py,
             done = n_turns;  // every particle is lost; nothing left to write
             break;
         }
-        if (cancel_requested()) {
+        if (!wait || cancel_requested()) {
             // Flush the survivors with their current steps and stop.
             c.turn0 = inverse ? s0 - done : s0 + done;
             c.n_turns = 0;
