@@ -442,8 +442,10 @@ __device__ __forceinline__ float hi_max(float m, double a, double b) {
 // per scheduler.
 constexpr uint32_t kBlockTurns = 16u;
 
+// EVERY looks at every turn: for orbits that reach t but stay below
+// Barrier::small_hi, the bound then.
 // Returns the pattern to compare with the bound (below it: nothing lost).
-template <int ARITH, bool OCT, bool REV, int K>
+template <int ARITH, bool OCT, bool REV, int K, bool EVERY = false>
 __device__ __forceinline__ uint32_t block_turns(Particle (&p)[K], const double2 *q, double mu) {
     constexpr int D = REV ? -2 : 2;
     constexpr int kUnroll = K <= 2 ? int(kBlockTurns) : 4;
@@ -454,7 +456,8 @@ __device__ __forceinline__ uint32_t block_turns(Particle (&p)[K], const double2 
 #pragma unroll
         for (int j = 0; j < K; ++j) {
             turn<ARITH, OCT, REV>(p[j], Turn{a.x, a.y, b.x, b.y}, mu);
-            if (u & 1) big = hi_max(hi_max(big, p[j].x, p[j].px), p[j].y, p[j].py);
+            if (EVERY || (u & 1))
+                big = hi_max(hi_max(big, p[j].x, p[j].px), p[j].y, p[j].py);
         }
     }
     return __float_as_uint(big) & 0x7fffffffu;

@@ -135,7 +135,8 @@ __device__ __forceinline__ Turn staged_record(const double *rec, uint32_t kn, ui
 // and applies the block's turns.  If the coordinates looked at stayed below
 // the bound, no particle can have been lost in the block, which is then
 // exactly what the per-turn test would have produced.  Otherwise the warp
-// restores the saved particles and redoes the block with the per-turn test
+// restores the saved particles and redoes the block: looking at every turn,
+// whose bound is higher, if that may still pass, else with the per-turn test
 // (turn_all).  The warp votes on a block while it already runs the next one
 // (hence two checkpoints): a vote before each block made every warp wait
 // for the end of its chain of turns, 54 instead of 50 cycles a turn with one
@@ -143,6 +144,27 @@ __device__ __forceinline__ Turn staged_record(const double *rec, uint32_t kn, ui
 // a loss cheap (at most 32 turns repeated) where a fifth of the particles is
 // lost in 512 turns; blocks of 8 cost 1.4 cycles a turn more and runs of 128
 // turns 4 % of the dynamic-aperture scan.
+//
+// A small barrier has orbits that live above a bound (at mu = 0 that of every
+// second turn is 1.35 for barrier 10, 0.50 for 2 and 0.31 for 1, that of every
+// turn half the barrier): after kVainRedos blocks of a stage that were redone
+// for nothing the warp looks, or tests, that way for the rest of the stage.
+// One such block is more often an orbit on its way out.  ms for 10^4 turns,
+// with per-turn looks in runs of 32, with blocks that were all retested, now:
+//     barrier             0.8    1      2      3      10
+//     90,000 particles    4.16   4.52   4.07   4.05   2.02
+//       (mu = 0.2)        5.75   5.61   4.73   4.24   1.87
+//                         3.10   3.11   2.19   2.03   1.82
+//     3,600 particles     2.22   1.94   1.74   1.75   0.47
+//       (mu = 0)          2.42   2.12   1.76   0.56   0.33
+//                         1.91   1.51   0.40   0.35   0.33
+enum class Look {
+    kPairs,  // at every second turn
+    kEvery,  // at every turn
+    kTest,   // the test itself
+};
+constexpr uint32_t kVainRedos = 2;
+
 // Returns false when a copy did not land within the bounded wait (the
 // chunk's results are then invalid and c.fault is set).
 template <int ARITH, bool OCT, bool REV, int K>
@@ -195,13 +217,13 @@ __device__ __forceinline__ bool turns_staged(const TrackChunk &c, const Barrier 
         if (!timed_out) {
             // A caller's records are checked to be rotations, which the
             // test of every second turn needs.
-            bool pairs = c.pair_hi != 0u;
-            if (pairs && c.check_records) {
+            Look look = c.pair_hi != 0u ? Look::kPairs : Look::kEvery;
+            if (look == Look::kPairs && c.check_records) {
                 const double2 *q = reinterpret_cast<const double2 *>(rec);
                 bool unit = true;
                 for (uint32_t kk = threadIdx.x & 31u; kk < kn; kk += 32u)
                     unit = unit && dev::is_rotation(q[2u * kk], q[2u * kk + 1u]);
-                pairs = __all_sync(kFullMask, unit);
+                if (!__all_sync(kFullMask, unit)) look = Look::kEvery;
             }
             constexpr uint32_t B = dev::kBlockTurns;
             const uint32_t pair_hi = c.pair_hi;
@@ -222,44 +244,87 @@ __device__ __forceinline__ bool turns_staged(const TrackChunk &c, const Barrier 
                 save = saved;
                 saved = t;
             };
-            bool check = false;  // this thread's verdict on the block before
-            for (uint32_t j0 = 0; warp_live && j0 < kn;) {
-                bool again = false;  // the warp's
-                // The hot loop holds nothing but blocks: with the redo's code
-                // inside it a turn took 3 cycles more.
-                const uint32_t jb = pairs ? j0 + (kn - j0) / B * B : j0;
-                const double2 *q = record(j0);
-#pragma unroll 2
-                for (; j0 < jb; j0 += B, q += REV ? -int(2u * B) : int(2u * B)) {
-                    checkpoint();
-                    again = __any_sync(kFullMask, check);
-                    const bool next = dev::block_turns<ARITH, OCT, REV, K>(p, q, mu) >= pair_hi;
-                    if (again) break;
-                    check = next;
-                    swap();
+            auto restore = [&]() {
+#pragma unroll
+                for (int j = 0; j < K; ++j) {
+                    const double2 *const from = saved + 2u * (j * blockDim.x + threadIdx.x);
+                    const double2 a = from[0], b = from[1];
+                    p[j] = dev::make_particle(a.x, a.y, b.x, b.y);
                 }
-                if (!again && j0 < kn) {  // a short block, or records of another kind
+            };
+            bool check = false;  // this thread's verdict on the block before ...
+            uint32_t top = 0u;   // ... and the largest coordinate it saw
+            uint32_t soft = 0u, vain = 0u;  // blocks redone without a loss, by the two tests
+            for (uint32_t j0 = 0; warp_live && j0 < kn;) {
+                if (look == Look::kTest) {
+                    for (; warp_live && j0 < kn; ++j0)
+                        turn_all<ARITH, OCT, REV, K>(c, bar, mu, staged_record(rec, kn, j0, REV),
+                                                     k0 + j0, p, id, live, warp_live);
+                    break;
+                }
+                bool again = false;  // the warp's
+                // The hot loops hold nothing but blocks: with the redo's code
+                // inside a turn took 3 cycles more.
+                const uint32_t jb = j0 + (kn - j0) / B * B;
+                const double2 *q = record(j0);
+                if (look == Look::kPairs) {
+#pragma unroll 2
+                    for (; j0 < jb; j0 += B, q += REV ? -int(2u * B) : int(2u * B)) {
+                        checkpoint();
+                        again = __any_sync(kFullMask, check);
+                        const uint32_t seen = dev::block_turns<ARITH, OCT, REV, K>(p, q, mu);
+                        if (again) break;
+                        check = seen >= pair_hi;
+                        top = seen;
+                        swap();
+                    }
+                } else {
+#pragma unroll 1
+                    for (; j0 < jb; j0 += B, q += REV ? -int(2u * B) : int(2u * B)) {
+                        checkpoint();
+                        again = __any_sync(kFullMask, check);
+                        const uint32_t seen = dev::block_turns<ARITH, OCT, REV, K, true>(p, q, mu);
+                        if (again) break;
+                        check = seen >= bar.small_hi;
+                        top = seen;
+                        swap();
+                    }
+                }
+                if (!again && j0 < kn) {  // a short block
                     checkpoint();
                     again = __any_sync(kFullMask, check);
                     if (!again) {
-                        check = dev::each_turn<ARITH, OCT, REV, K>(p, record(j0), min(B, kn - j0),
-                                                                   mu) >= bar.small_hi;
+                        top = dev::each_turn<ARITH, OCT, REV, K>(p, record(j0), kn - j0, mu);
+                        check = top >= bar.small_hi;
                         j0 += B;
                         swap();
                     }
                 }
                 if (!again && j0 >= kn) again = __any_sync(kFullMask, check);
-                if (again) {  // the block that ended at j0, turn by turn
-#pragma unroll
-                    for (int j = 0; j < K; ++j) {
-                        const double2 *const from = saved + 2u * (j * blockDim.x + threadIdx.x);
-                        const double2 a = from[0], b = from[1];
-                        p[j] = dev::make_particle(a.x, a.y, b.x, b.y);
+                if (again) {  // the block that ended at j0
+                    restore();
+                    bool test = __any_sync(kFullMask, top >= bar.small_hi);
+                    if (!test) {
+                        // Above the bound of every second turn alone.
+                        top = dev::each_turn<ARITH, OCT, REV, K>(p, record(j0 - B), B, mu);
+                        test = __any_sync(kFullMask, top >= bar.small_hi);
+                        if (test) restore();
+                        else if (++soft == kVainRedos) look = Look::kEvery;
                     }
-                    const uint32_t j1 = min(j0, kn);
-                    for (uint32_t kk = j0 - B; warp_live && kk < j1; ++kk)
-                        turn_all<ARITH, OCT, REV, K>(c, bar, mu, staged_record(rec, kn, kk, REV),
-                                                     k0 + kk, p, id, live, warp_live);
+                    if (test) {  // turn by turn
+                        const uint32_t j1 = min(j0, kn);
+                        int was = 0, is = 0;  // this thread's live particles
+#pragma unroll
+                        for (int j = 0; j < K; ++j) was += live[j] ? 1 : 0;
+                        for (uint32_t kk = j0 - B; warp_live && kk < j1; ++kk)
+                            turn_all<ARITH, OCT, REV, K>(c, bar, mu,
+                                                         staged_record(rec, kn, kk, REV), k0 + kk,
+                                                         p, id, live, warp_live);
+#pragma unroll
+                        for (int j = 0; j < K; ++j) is += live[j] ? 1 : 0;
+                        if (!__any_sync(kFullMask, was != is) && ++vain == kVainRedos)
+                            look = Look::kTest;
+                    }
                     check = false;
                 }
             }
