@@ -307,6 +307,32 @@ Workspace carve(void *base, size_t n) {
 // millisecond of exact turns at the full rate, 6 ms with kicks.
 constexpr uint64_t kMaxInFlight = uint64_t(1) << 29;
 
+// Turns of a one-chunk call from which staged records and blocks of turns are
+// faster than direct reads with twice the warps per SM.  A list that the
+// staged kernel holds at once (four warps per scheduler) gains from the first
+// block of 16 turns on; a longer one runs in waves, and with the octupole the
+// FP64 pipe is nearly full in both.  us, direct and staged:
+//     particles   16 turns      32            64            128
+//     mu = 0
+//        40,000   5.5   4.1     9.1   5.9     16.4  10.2    30.0  17.4
+//        90,000   6.0   6.2     9.7   8.7     17.3  14.7    32.4  25.6
+//       262,144   9.6  11.7    16.7  17.5     30.5  30.3    57.4  54.6
+//       640,000  19.9  25.1    35.9  36.2     67.2  62.5   127.5 115.2
+//     mu = 0.2
+//        10,000   5.3   4.0     8.9   6.5     15.9  10.0
+//        40,000   5.5   5.8     9.3   9.8     16.5  16.0    31.1  25.7
+//        90,000   6.7   7.9    11.3  12.9     20.2  21.9    37.6  37.9
+//       262,144  13.1  16.0    23.6  25.5     43.7  46.6    83.0  84.2
+//       640,000  27.9  33.9    51.5  52.9     97.7  98.3   185.8 183.9
+// Fast arithmetic has fewer FP64 instructions: with the octupole 5.5 and 5.1
+// us for 16 turns of 40,000 particles, 118.4 and 113.7 for 64 of 1,048,576.
+uint32_t stage_from_turns(size_t n, bool octupole, hm_arith arith) {
+    const size_t warps = n / (size_t(sm_count()) * 128u);  // full ones per scheduler
+    if (!octupole) return warps < 4u ? 16u : (warps < 8u ? 24u : 40u);
+    if (arith == HM_ARITH_FAST) return warps < 3u ? 16u : 64u;
+    return warps < 1u ? 16u : (warps < 3u ? 48u : 112u);
+}
+
 }  // namespace
 
 // Advances n particles by n_turns turns of the map; *turns_done receives
@@ -351,7 +377,6 @@ hm_status track_driver(double *x, double *px, double *y, double *py,
     c.b2bits = b2bits;
     c.kick_module = kick_module;
     c.kick_seed = kick_seed;
-    c.pair_hi = pair_threshold_hi(b2, mu);
     c.check_records = !own_table;
     TrackLaunch l{int(arith), mu != 0.0, inverse, cfg.per_thread, cfg.threads};
 
@@ -363,14 +388,16 @@ hm_status track_driver(double *x, double *px, double *y, double *py,
     // Staged turn records need a table that double2 loads and bulk copies can
     // read (16-byte aligned), and the bulk copies the workspace's fault word.
     // A call of one chunk stages all its records at once, without bulk
-    // copies; below 16 turns the direct reads are as quick.
+    // copies, from stage_from_turns on.
     const bool stageable = cfg.stage_turns != 0 && (reinterpret_cast<uintptr_t>(table) & 15u) == 0;
     const bool staged = stageable && !one_chunk;
     c.stage_turns = staged ? cfg.stage_turns : 0u;
-    if (stageable && one_chunk && n_turns >= 16u && n_turns <= 512u) {
+    if (stageable && one_chunk && n_turns <= 512u &&
+        n_turns >= stage_from_turns(n, mu != 0.0, arith)) {
         c.stage_turns = 16u;
         while (c.stage_turns < n_turns) c.stage_turns *= 2u;
     }
+    if (c.stage_turns != 0u) c.pair_hi = pair_threshold_hi(b2, mu);
     c.fault = staged ? w.fault : nullptr;
     if (staged) HM_CUDA_TRY(cudaMemsetAsync(w.fault, 0, sizeof(uint32_t), stream));
 

@@ -17,6 +17,7 @@
 // henon_tracker_gpu::track, src/henon.cu:3155-3185.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <atomic>
 #include <cstdint>
 
@@ -627,9 +628,11 @@ __device__ __forceinline__ void track_chunk(const TrackChunk &c) {
 //     exact, mu = 0      56.4  48.4  45.5  44.3   (before: 69.9  53.2  50.9  48.9)
 //     exact, mu != 0     80.7  74.8  72.7  71.6   (before: 91.9  79.9  76.4  74.6)
 // Before: per-turn looks, runs of 32 turns, 64 registers.  With 64 registers
-// the blocks of turns took 68.3, 48.8, 47.1 and 44.9 at mu = 0.
+// the blocks of turns took 68.3, 48.8, 47.1 and 44.9 at mu = 0.  The kernels
+// that read the records from global memory run a few turns: 64 registers,
+// for twice the loads in flight.
 template <int ARITH, bool OCT, bool REV, int K, bool STAGED>
-__global__ void __launch_bounds__(256, K <= 2 ? 2 : 1) track_chunk_kernel(const TrackChunk c) {
+__global__ void __launch_bounds__(256, K <= 2 ? (STAGED ? 2 : 4) : 1) track_chunk_kernel(const TrackChunk c) {
     track_chunk<ARITH, OCT, REV, K, STAGED, false>(c);
 }
 
@@ -682,14 +685,24 @@ cudaError_t launch_k(const TrackChunk &c, const TrackLaunch &l, uint32_t n_upper
     // the device is full; a short list would instead leave SMs idle (a
     // particle is one serial chain of turns whatever its thread holds), so
     // K is halved while the grid would give fewer than two blocks per SM.
-    int K = l.per_thread;
-    const uint64_t min_blocks = kMinBlocksPerSm * uint64_t(sm_count());
+    // A launch that reads its records from global memory runs few turns and
+    // waits for its loads: at least two particles per thread then, from
+    // three blocks per SM on (us for 8 turns with one and two, mu = 0:
+    // 90,000 particles 4.1 and 4.3, 262,144 7.6 and 6.2, 1,048,576 23.7 and
+    // 18.3; for 16 turns at mu = 0.2: 6.7 / 7.2, 14.9 / 13.1, 51.2 / 43.9).
+    const bool direct = c.stage_turns == 0;
+    int K = direct ? std::max(l.per_thread, 2) : l.per_thread;
+    const uint64_t sms = uint64_t(sm_count());
+    const uint64_t min_blocks = kMinBlocksPerSm * sms;
+    const uint64_t pair_blocks = direct ? 3u * sms : min_blocks;
     while (K > 1 && (uint64_t(n_upper) + uint64_t(threads) * K - 1) / (uint64_t(threads) * K) <
-                        min_blocks)
+                        pair_blocks)
         K /= 2;
     // Likewise smaller blocks: they spread a short list more evenly (40,000
-    // particles in blocks of 128 give some SMs three blocks, most two).
-    while (threads > 32 && threads % 64 == 0 &&
+    // particles in blocks of 128 give some SMs three blocks, most two).  A
+    // few turns do not pay for starting more SMs (1,024 particles, one turn:
+    // 2.1 us in blocks of 32, 1.8 in blocks of 128).
+    while (!direct && threads > 32 && threads % 64 == 0 &&
            (uint64_t(n_upper) + uint64_t(threads) * K - 1) / (uint64_t(threads) * K) < min_blocks)
         threads /= 2;
     const uint64_t per_block = uint64_t(threads) * uint64_t(K);

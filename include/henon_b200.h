@@ -97,8 +97,9 @@ typedef int (*hm_cancel_fn)(void *ctx);
 hm_status hm_set_cancel_callback(hm_cancel_fn fn, void *ctx);
 
 /* Launch shape of the chunked tracking kernels: threads per block (32..256,
- * multiple of 32), particles per thread (1, 2 or 4), turns of the first
- * chunk and the cap of the doubling chunk length.  Process-wide; chosen by
+ * multiple of 32), particles per thread (1, 2 or 4; fewer on short lists,
+ * at least two on long ones whose records are read directly), turns of the
+ * first chunk and the cap of the doubling chunk length.  Process-wide; chosen by
  * the autotuner.  Results do not depend on it. */
 hm_status hm_set_track_config(int threads, int per_thread, uint32_t chunk0,
                               uint32_t chunk_max);
@@ -110,8 +111,8 @@ hm_status hm_get_track_config(int *threads, int *per_thread,
  * of records at a time into shared memory with a bulk copy (TMA,
  * double-buffered, bounded waits) and every warp reads them from there.
  * stage_turns is 0 or a power of two in [16, 512] (default 512); a run of
- * less than 16 turns uses direct reads.  Process-wide; results do not
- * depend on it.
+ * less than 16 turns, and one of up to 112 on a large set, uses direct
+ * reads.  Process-wide; results do not depend on it.
  * A staged copy that does not land within its bounded wait makes the call
  * return HM_ERR_TIMEOUT.  After HM_ERR_TIMEOUT the particles' coordinates
  * and steps are unspecified (the chunk that gave up may have moved some of
