@@ -358,7 +358,7 @@ __device__ __forceinline__ bool turns_staged(const TrackChunk &c, const Barrier 
 // The kicks do not depend on the orbit, so a warp makes those of kKickTurns
 // turns of its 32 particles together and then runs the turns.  Each kick
 // takes the first point of each of two attempts' sequences that lies in the
-// unit disc (dev::kick_direction), 1.6 Philox blocks on average; with the
+// unit disc (dev::kick_direction), 1.5 Philox blocks on average; with the
 // rejection loop inside the turn a warp waited for its slowest lane, 3.6
 // blocks a turn.  Here every lane makes the first attempt of its own kicks,
 // the rejected ones (38 %) go to a list, and each further attempt is made for
@@ -367,11 +367,16 @@ __device__ __forceinline__ bool turns_staged(const TrackChunk &c, const Barrier 
 // 262,144 particles x 2,000 turns, mu = 0.2: 10.0 ms before, 6.4 now, 66 % of
 // the issue slots and 37 % of the FP64 pipe busy; 299 instructions per warp
 // and turn (421 before), about half of them the generator's.  Groups of 4
-// turns 7.5 ms, of 16 6.8 (fewer warps fit).
+// turns 7.5 ms, of 16 6.8 (fewer warps fit).  A last group of fewer turns
+// makes their kicks only (9 turns of 262,144 particles 49.7 -> 38.9 us).
 //
 // Shared memory of a warp: the points (then the kicks) of its turns, the list,
 // the particles' indices and the turns' records.
 constexpr uint32_t kKickTurns = 8;
+// Turns of a chunk from which groups pay: a single turn's kicks are made by
+// each lane for itself (262,144 particles, us for one turn: 9.3 so, 11.8 as a
+// group of one; for two turns 14.8 as a group, 14.5 so).
+constexpr uint32_t kKickGroup = 2;
 
 struct KickShared {
     double2 a[kKickTurns * 32], b[kKickTurns * 32];  // {u1, u2}, {u3, u4} of [turn][lane]
@@ -402,18 +407,24 @@ __device__ __forceinline__ void make_kicks(KickShared &w, const TrackChunk &c, u
     const unsigned lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
     const uint32_t k0 = uint32_t(c.kick_seed), k1 = uint32_t(c.kick_seed >> 32);
     uint32_t n_list = 0;
-#pragma unroll 4
-    for (uint32_t u = 0; u < kKickTurns; ++u) {
+    auto first = [&](uint32_t u) {
         const uint32_t slot = u * 32u + lane;
         // what kick_direction falls back to when no attempt gives a point
         w.a[slot] = make_double2(0.0, 0.0);
         w.b[slot] = make_double2(1.0, 0.0);
         const uint32_t got =
             kick_attempt(k0, k1, id, t0 + uint32_t(int(u) * dt), 0u, 0u, &w.a[slot], &w.b[slot]);
-        const bool more = live && u < kn && got != 3u;
+        const bool more = live && got != 3u;
         const unsigned m = __ballot_sync(kFullMask, more);
         if (more) w.list[n_list + __popc(m & below)] = uint16_t(slot | (got << 14));
         n_list += __popc(m);
+    };
+    if (kn == kKickTurns) {
+#pragma unroll 4
+        for (uint32_t u = 0; u < kKickTurns; ++u) first(u);
+    } else {
+#pragma unroll 1
+        for (uint32_t u = 0; u < kn; ++u) first(u);
     }
     for (uint32_t at = 1; n_list > 0u && at < dev::kKickAttempts; ++at) {
         __syncwarp();
@@ -440,14 +451,20 @@ __device__ __forceinline__ void make_kicks(KickShared &w, const TrackChunk &c, u
     __syncwarp();
     // (u1, u2, u3 f, u4 f), f = sqrt((1 - s1) / s2), times the module
     const double km = c.kick_module;
-#pragma unroll 4
-    for (uint32_t u = 0; u < kKickTurns; ++u) {
+    auto scale = [&](uint32_t u) {
         const double2 a = w.a[u * 32u + lane], b = w.b[u * 32u + lane];
         const double s1 = Rn::add(Rn::mul(a.x, a.x), Rn::mul(a.y, a.y));
         const double s2 = Rn::add(Rn::mul(b.x, b.x), Rn::mul(b.y, b.y));
         const double f = __dsqrt_rn(Rn::div(Rn::sub(1.0, s1), s2));
         w.a[u * 32u + lane] = make_double2(Rn::mul(a.x, km), Rn::mul(a.y, km));
         w.b[u * 32u + lane] = make_double2(Rn::mul(Rn::mul(b.x, f), km), Rn::mul(Rn::mul(b.y, f), km));
+    };
+    if (kn == kKickTurns) {
+#pragma unroll 4
+        for (uint32_t u = 0; u < kKickTurns; ++u) scale(u);
+    } else {
+#pragma unroll 1
+        for (uint32_t u = 0; u < kn; ++u) scale(u);
     }
 }
 
@@ -463,6 +480,31 @@ __device__ __forceinline__ void add_kick(Particle &p, double2 a, double2 b) {
     }
 }
 
+// Particle `id`, lost in turn k of the chunk.
+template <bool REV>
+__device__ __forceinline__ void lose(const TrackChunk &c, uint32_t id, bool &live, uint32_t k) {
+    c.ux[id] = quiet_nan();
+    c.upx[id] = quiet_nan();
+    c.uy[id] = quiet_nan();
+    c.upy[id] = quiet_nan();
+    c.usteps[id] = REV ? c.turn0 - k : c.turn0 + k;
+    live = false;
+}
+
+// A chunk of fewer than kKickGroup turns with kicks: each lane makes its own.
+template <int ARITH, bool OCT, bool REV>
+__device__ __forceinline__ void turns_kicked_few(const TrackChunk &c, const Barrier &bar,
+                                                 Particle &p, uint32_t id, bool &live) {
+    for (uint32_t k = 0; live && k < c.n_turns; ++k) {
+        const uint32_t t = REV ? c.turn0 - 1u - k : c.turn0 + k;
+        const dev::KickDirection d = dev::kick_direction(c.kick_seed, id, t);
+        if (!REV) dev::apply_kick<false>(p, d, c.kick_module);
+        dev::turn<ARITH, OCT, REV>(p, dev::load_turn(c.table, t), c.mu);
+        if (REV) dev::apply_kick<true>(p, d, c.kick_module);
+        if (!dev::inside_after_turn<ARITH>(p, bar)) lose<REV>(c, id, live, k);
+    }
+}
+
 // The chunk's turns with kicks (one particle per thread): groups of
 // kKickTurns turns, redone with the per-turn test where a live particle's
 // coordinate reached the bound.  A lost particle's registers move with the
@@ -471,10 +513,10 @@ template <int ARITH, bool OCT, bool REV>
 __device__ __forceinline__ void turns_kicked(const TrackChunk &c, const Barrier &bar,
                                              Particle &p, uint32_t id, bool &live,
                                              bool warp_live) {
+    const double mu = c.mu;
     extern __shared__ __align__(128) double stage_buf[];
     KickShared &w = reinterpret_cast<KickShared *>(stage_buf)[threadIdx.x >> 5];
     const unsigned lane = threadIdx.x & 31u;
-    const double mu = c.mu;
     w.id[lane] = id;
     auto turn = [&](uint32_t u) {
         const double2 a = w.a[u * 32u + lane], b = w.b[u * 32u + lane];
@@ -514,14 +556,7 @@ __device__ __forceinline__ void turns_kicked(const TrackChunk &c, const Barrier 
             p = from;
             for (uint32_t u = 0; u < kn; ++u) {
                 turn(u);
-                if (live && !dev::inside_after_turn<ARITH>(p, bar)) {
-                    c.ux[id] = quiet_nan();
-                    c.upx[id] = quiet_nan();
-                    c.uy[id] = quiet_nan();
-                    c.upy[id] = quiet_nan();
-                    c.usteps[id] = REV ? c.turn0 - k0 - u : c.turn0 + k0 + u;
-                    live = false;
-                }
+                if (live && !dev::inside_after_turn<ARITH>(p, bar)) lose<REV>(c, id, live, k0 + u);
             }
             warp_live = __any_sync(kFullMask, live);
         }
@@ -575,7 +610,11 @@ __device__ __forceinline__ void track_chunk(const TrackChunk &c) {
     const bool warp_live = __any_sync(kFullMask, thread_live);
     if constexpr (KICK) {
         static_assert(K == 1, "kicked turns run one particle per thread");
-        turns_kicked<ARITH, OCT, REV>(c, bar, p[0], id[0], live[0], warp_live);
+        // STAGED: the kicks of a group of turns in shared memory
+        if constexpr (STAGED)
+            turns_kicked<ARITH, OCT, REV>(c, bar, p[0], id[0], live[0], warp_live);
+        else
+            turns_kicked_few<ARITH, OCT, REV>(c, bar, p[0], id[0], live[0]);
     } else if (STAGED) {
         if (!turns_staged<ARITH, OCT, REV, K>(c, bar, p, id, live, warp_live)) return;
     } else {
@@ -640,6 +679,11 @@ __global__ void __launch_bounds__(256, K <= 2 ? (STAGED ? 2 : 4) : 1) track_chun
 // (with 96, five: 6.74 against 6.40 ms).
 template <int ARITH, bool OCT, bool REV>
 __global__ void __launch_bounds__(256, 3) track_kicked_kernel(const TrackChunk c) {
+    track_chunk<ARITH, OCT, REV, 1, true, true>(c);
+}
+
+template <int ARITH, bool OCT, bool REV>
+__global__ void __launch_bounds__(256, 4) track_kicked_few_kernel(const TrackChunk c) {
     track_chunk<ARITH, OCT, REV, 1, false, true>(c);
 }
 
@@ -674,6 +718,10 @@ cudaError_t launch_k(const TrackChunk &c, const TrackLaunch &l, uint32_t n_upper
     if (!isnan(c.kick_module)) {
         const unsigned blocks = unsigned((uint64_t(n_upper) + threads - 1) / threads);
         if (blocks == 0) return cudaSuccess;
+        if (c.n_turns < kKickGroup) {
+            track_kicked_few_kernel<ARITH, OCT, REV><<<blocks, threads, 0, s>>>(c);
+            return cudaGetLastError();
+        }
         const size_t smem = size_t(threads / 32) * sizeof(KickShared);
         auto kernel = track_kicked_kernel<ARITH, OCT, REV>;
         const cudaError_t e = allow_smem(kernel, smem);
