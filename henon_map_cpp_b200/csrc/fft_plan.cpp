@@ -30,9 +30,9 @@ namespace {
 using cld = std::complex<long double>;
 
 // Radices of M: fives and threes first (the early stages, whose spans are
-// long), then the power of two in as few stages as radix 16 allows, of about
-// equal radices (2^13 = 16 8 8 8), the larger first; false when M has
-// another prime factor.
+// long), then the power of two in as few stages as radix 16 (short rows: 8)
+// allows, of about equal radices (2^13 = 16 8 8 8), the larger first; false
+// when M has another prime factor.
 bool factor(uint32_t M, std::vector<uint8_t> *rad) {
     rad->clear();
     uint32_t m = M;
@@ -43,7 +43,8 @@ bool factor(uint32_t M, std::vector<uint8_t> *rad) {
         }
     int bits = 0;
     for (; m % 2 == 0; m /= 2) ++bits;
-    for (int left = (bits + 3) / 4; left > 0; --left) {
+    const int most = M >= kFftLongRow ? 4 : 3;  // bits of the largest radix
+    for (int left = (bits + most - 1) / most; left > 0; --left) {
         const int b = (bits + left - 1) / left;
         rad->push_back(uint8_t(1 << b));
         bits -= b;

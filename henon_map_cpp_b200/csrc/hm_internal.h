@@ -489,12 +489,15 @@ cudaError_t launch_fft_peak2(const double2 *z, uint32_t len, size_t n, uint32_t 
                              cudaStream_t s);
 // FFT tunes of one window computed whole in one block's shared memory
 // (tunes.cu; plans in fft_plan.cpp): the DFT of the window's L samples is
-// an in-place mixed-radix network of length M (radices 2, 3, 4, 5, 8) when L
+// an in-place mixed-radix network of length M (radices 2, 3, 4, 5, 8, 16) when L
 // has no other prime factor (M = L), else Bluestein's chirp convolution
 // with M >= 2L - 1.  M is at most kFftMaxLen (the row fills at most 200 KB
 // of shared memory); longer windows take the library path above.
 constexpr int kFftMaxStages = 24;
 constexpr uint32_t kFftMaxLen = 12800;
+// Transform length from which two rows no longer fit in an SM's shared memory:
+// radix 16 and the long rows' kernel (tunes.cu) from here on.
+constexpr uint32_t kFftLongRow = 7040;
 struct FftPlanDev {
     uint32_t L = 0, M = 0;
     int bluestein = 0;

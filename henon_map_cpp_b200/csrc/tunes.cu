@@ -27,6 +27,7 @@
 
 #include <algorithm>
 #include <cstdint>
+#include <type_traits>
 
 #include "hm_device.cuh"
 #include "hm_internal.h"
@@ -629,14 +630,13 @@ __global__ void fft_peak_kernel(const double2 *buf, uint32_t len, size_t count,
 // interpolation depends on magnitude ratios only, so the peak is taken on
 // |conv_k| directly.
 //
-// A row's time is its passes over shared memory with a barrier after each, so
-// there are as few as possible: radix 16 where the power of two allows; the
+// A long row's time is its passes over shared memory with a barrier after each,
+// so there are as few as possible: radix 16 where the power of two allows; the
 // first stage takes its values from the orbit; Bluestein's last forward stage,
 // the product and the first inverse stage, which work on the same values,
 // are one pass; the last stage looks for the maximum as it writes.  2^13
-// values: 8 passes instead of 13.  32,768 rows, before -> now: windows of 1001
-// (M = 2048) 1.16 -> 1.03 ms, 4001 (8192) 6.67 -> 5.33, 5001 (10240) 7.91 ->
-// 6.6, 10,000 (direct) 6.1 -> 6.2; 38-41 % of the issue slots and 24-37 % of the
+// values: 8 passes instead of 13.  32,768 rows, before -> now: windows of 4001
+// (M = 8192) 6.67 -> 5.33 ms, 5001 (10240) 7.91 -> 6.6, 10,000 (direct) 6.1 -> 6.2; 38-41 % of the issue slots and 24-37 % of the
 // FP64 pipe busy: one row fills an SM, so its passes, arithmetic and reads
 // of the orbit follow one another.
 
@@ -798,25 +798,36 @@ __device__ __forceinline__ uint32_t slot(uint32_t i) {
 }
 
 // The twiddles w^k, k < R, w = exp(-2 pi i t / M): w, w^4 and w^8 from the
-// tables, the others at most three products from those.
+// tables, the others at most three products from those.  Radix 8 makes
+// w^5 .. w^7 as it uses them: with all of them in registers beside its eight
+// values the short rows' kernel spilled.
 template <int R>
-__device__ __forceinline__ void twiddles(double2 (&w)[R], const double2 *tc, const double2 *tf,
-                                         uint32_t t) {
-    w[0] = make_double2(1.0, 0.0);
-    w[1] = fft_twiddle(tc, tf, t);
-    if constexpr (R > 2) w[2] = c_mul(w[1], w[1]);
-    if constexpr (R > 3) w[3] = c_mul(w[1], w[2]);
-    if constexpr (R > 4) w[4] = R > 5 ? fft_twiddle(tc, tf, 4u * t) : c_mul(w[2], w[2]);
-    if constexpr (R > 5) {
+struct Twiddles {
+    static constexpr int kKept = R == 8 ? 5 : R;
+    double2 w[kKept];
+    __device__ __forceinline__ Twiddles(const double2 *tc, const double2 *tf, uint32_t t) {
+        w[0] = make_double2(1.0, 0.0);
+        w[1] = fft_twiddle(tc, tf, t);
+        if constexpr (R > 2) w[2] = c_mul(w[1], w[1]);
+        if constexpr (R > 3) w[3] = c_mul(w[1], w[2]);
+        if constexpr (R > 4) w[4] = R > 5 ? fft_twiddle(tc, tf, 4u * t) : c_mul(w[2], w[2]);
+        if constexpr (R > 8) {
 #pragma unroll
-        for (int k = 5; k < 8; ++k) w[k] = c_mul(w[4], w[k - 4]);
-    }
-    if constexpr (R > 8) {
-        w[8] = fft_twiddle(tc, tf, 8u * t);
+            for (int k = 5; k < 8; ++k) w[k] = c_mul(w[4], w[k - 4]);
+            w[8] = fft_twiddle(tc, tf, 8u * t);
 #pragma unroll
-        for (int k = 9; k < 16; ++k) w[k] = c_mul(w[8], w[k - 8]);
+            for (int k = 9; k < 16; ++k) w[k] = c_mul(w[8], w[k - 8]);
+        }
     }
-}
+    __device__ __forceinline__ double2 pow(int k) const {
+        if constexpr (R == 8) return k < 5 ? w[k] : c_mul(w[4], w[k - 4]);
+        else return w[k];
+    }
+};
+
+struct NoTwiddles {
+    __device__ __forceinline__ NoTwiddles(const double2 *, const double2 *, uint32_t) {}
+};
 
 // First maximum of |X_k|^2 (monotone in |X_k|), ties to the smallest k.
 struct Peak {
@@ -878,20 +889,20 @@ __device__ __forceinline__ void fft_stage(const FftRow &r, uint32_t span, uint32
                                           Peak &peak) {
     double2 *const row = r.row;
     butterflies<R>(r, span, [&](uint32_t j, uint32_t base) {
-        double2 v[R], w[R];
-        if constexpr (TW) twiddles<R>(w, r.tc, r.tf, j * prod);
+        double2 v[R];
+        const std::conditional_t<TW, Twiddles<R>, NoTwiddles> w(r.tc, r.tf, j * prod);
 #pragma unroll
         for (int q = 0; q < R; ++q) {
             if constexpr (MODE == kFromOrbit) v[q] = in(base + q * span);
             else v[q] = row[slot<SWZ>(base + q * span)];
             if constexpr (TW && INV)
-                if (q > 0) v[q] = c_mulc(v[q], w[q]);
+                if (q > 0) v[q] = c_mulc(v[q], w.pow(q));
         }
         dft_small<R, INV>(v);
 #pragma unroll
         for (int k = 0; k < R; ++k) {
             if constexpr (TW && !INV)
-                if (k > 0) v[k] = c_mul(v[k], w[k]);
+                if (k > 0) v[k] = c_mul(v[k], w.pow(k));
             const uint32_t at = base + k * span;
             row[slot<SWZ>(at)] = v[k];
             if constexpr (MODE == kToPeak) {
@@ -912,11 +923,13 @@ __device__ __forceinline__ void fft_stage_any(const FftRow &r, uint32_t span, ui
     else fft_stage<R, INV, SWZ, true, MODE>(r, span, prod, in, peak);
 }
 
-template <bool INV, int SWZ, int MODE, class In>
+template <int MAXR, bool INV, int SWZ, int MODE, class In>
 __device__ void fft_stage_of(const FftRow &r, int s, In in, Peak &peak) {
     const uint32_t span = r.pl.stage_len[s], prod = r.pl.stage_prod[s];
     switch (r.pl.radix[s]) {
-        case 16: fft_stage_any<16, INV, SWZ, MODE>(r, span, prod, in, peak); break;
+        case 16:
+            if constexpr (MAXR >= 16) fft_stage_any<16, INV, SWZ, MODE>(r, span, prod, in, peak);
+            break;
         case 8: fft_stage_any<8, INV, SWZ, MODE>(r, span, prod, in, peak); break;
         case 4: fft_stage_any<4, INV, SWZ, MODE>(r, span, prod, in, peak); break;
         case 2: fft_stage_any<2, INV, SWZ, MODE>(r, span, prod, in, peak); break;
@@ -943,10 +956,12 @@ __device__ __forceinline__ void fft_turn(const FftRow &r) {
     }
 }
 
-template <int SWZ>
+template <int MAXR, int SWZ>
 __device__ void fft_turn_of(const FftRow &r) {
     switch (r.pl.radix[r.pl.n_stages - 1]) {
-        case 16: fft_turn<16, SWZ>(r); break;
+        case 16:
+            if constexpr (MAXR >= 16) fft_turn<16, SWZ>(r);
+            break;
         case 8: fft_turn<8, SWZ>(r); break;
         case 4: fft_turn<4, SWZ>(r); break;
         case 2: fft_turn<2, SWZ>(r); break;
@@ -955,15 +970,32 @@ __device__ void fft_turn_of(const FftRow &r) {
     }
 }
 
-// 512 threads of 128 registers: one radix-16 butterfly each for 8192 values.
-constexpr int kFftThreadsMax = 512;
+// Two kernels, by the length M of the transform.  Long rows (MAXR = 16, M >=
+// kFftLongRow): an SM's shared memory holds one of them, so the block has
+// few passes: 512 threads of 128 registers, one radix-16 butterfly each for
+// 8192 values, the first stage from the orbit, groups of threads.  Of shorter
+// rows (MAXR = 8) an SM holds several, whose passes overlap one another if
+// there are enough of them: radices to 8 in 64 registers, up to 256 threads
+// (at least 64), the row first brought into shared memory together with the
+// twiddles, one wait for both.  8,000 rows, us, with a pass for every step in 64
+// registers, with the long rows' kernel alone, and now:
+//     samples (M)       99 (200)  499 (1000)  1000   2999 (6000)  3071 (6144)   4800
+//     before             61          154       119       1147         1369       733
+//     long rows' kernel 127          216       206       1489         1234      1007
+//     now                63          179       124       1052          943       666
+// From M = 7200 on the long rows' kernel is the faster: 3,599 samples 1617 us,
+// with the other 1866.
 constexpr uint32_t kFftGroups = 4;
 
-template <int SWZ>
-__global__ void __launch_bounds__(kFftThreadsMax) fft_tune_kernel(const FftTuneArgs a) {
+template <int MAXR>
+constexpr int kFftThreadsMax = MAXR >= 16 ? 512 : 256;
+
+template <int MAXR, int SWZ>
+__global__ void __launch_bounds__(kFftThreadsMax<MAXR>, MAXR >= 16 ? 1 : 4)
+    fft_tune_kernel(const FftTuneArgs a) {
     extern __shared__ __align__(16) double2 fft_sm[];
-    __shared__ double red_m[kFftThreadsMax / 32];
-    __shared__ uint32_t red_k[kFftThreadsMax / 32];
+    __shared__ double red_m[kFftThreadsMax<MAXR> / 32];
+    __shared__ uint32_t red_k[kFftThreadsMax<MAXR> / 32];
     const FftPlanDev &pl = a.plan;
     double2 *row = fft_sm;
     double2 *tc = row + fft_row_slots(pl);
@@ -1001,7 +1033,7 @@ __global__ void __launch_bounds__(kFftThreadsMax) fft_tune_kernel(const FftTuneA
     }
     for (uint32_t t = threadIdx.x; t < pl.n_coarse; t += blockDim.x) tc[t] = pl.tw_coarse[t];
     for (uint32_t t = threadIdx.x; t < 64u; t += blockDim.x) tf[t] = pl.tw_fine[t];
-    __syncthreads();
+    if constexpr (MAXR >= 16) __syncthreads();
     const double *q = plane ? a.y : a.x, *p = plane ? a.py : a.px;
     const double mq = mean_of(a.means, a.n, i, 2 * plane, a.S);
     const double mp = mean_of(a.means, a.n, i, 2 * plane + 1, a.S);
@@ -1028,13 +1060,20 @@ __global__ void __launch_bounds__(kFftThreadsMax) fft_tune_kernel(const FftTuneA
     // arithmetic (8192 values, 32,768 rows: 5.38 instead of 5.62 ms).  Lengths
     // with fives keep them first: with 16 first and groups, 10240 values took
     // 7.27 ms instead of 6.49, their butterflies not dealing out evenly.
-    const bool split = last > 1 && pl.radix[0] % kFftGroups == 0;
+    const bool split = MAXR >= 16 && last > 1 && pl.radix[0] % kFftGroups == 0;
     const uint32_t groups = split ? kFftGroups : 1u;
-    const uint32_t per = blockDim.x / groups, group = threadIdx.x / per;
-    const FftRow part{pl,  row, tc, tf, group * (pl.M / groups), pl.M / groups,
-                      threadIdx.x - group * per, per};
+    const uint32_t per = MAXR >= 16 ? blockDim.x / groups : blockDim.x;
+    const uint32_t group = MAXR >= 16 ? threadIdx.x / per : 0u;
+    const FftRow part{pl,  row, tc, tf, MAXR >= 16 ? group * (pl.M / groups) : 0u,
+                      MAXR >= 16 ? pl.M / groups : pl.M,
+                      MAXR >= 16 ? threadIdx.x - group * per : threadIdx.x, per};
     static_assert(kFftGroups == 4u, "one named barrier per group below");
-    auto part_sync = [&]() {  // (barrier numbers as constants: five in all, not sixteen)
+    auto part_sync = [&]() {
+        if constexpr (MAXR < 16) {
+            __syncthreads();
+            return;
+        }
+        // (barrier numbers as constants: five in all, not sixteen)
         switch (group) {
             case 0: asm volatile("bar.sync 1, %0;" ::"r"(per) : "memory"); break;
             case 1: asm volatile("bar.sync 2, %0;" ::"r"(per) : "memory"); break;
@@ -1044,10 +1083,15 @@ __global__ void __launch_bounds__(kFftThreadsMax) fft_tune_kernel(const FftTuneA
     };
     Peak peak{-1.0, 0xffffffffu};
     int s = 0;  // forward stages done
-    if (last > 0) {
-        fft_stage_of<false, SWZ, kFromOrbit>(whole, 0, in, peak);
-        s = 1;
-    } else {
+    bool loaded = false;
+    if constexpr (MAXR >= 16)
+        if (last > 0) {
+            fft_stage_of<MAXR, false, SWZ, kFromOrbit>(whole, 0, in, peak);
+            s = 1;
+            loaded = true;
+        }
+    if (!loaded) {
+#pragma unroll 4
         for (uint32_t k = threadIdx.x; k < pl.M; k += blockDim.x) row[slot<SWZ>(k)] = in(k);
     }
     // Without first-NaN records the window's own samples decide
@@ -1059,24 +1103,24 @@ __global__ void __launch_bounds__(kFftThreadsMax) fft_tune_kernel(const FftTuneA
         return;
     }
     for (; s < last; ++s) {
-        fft_stage_of<false, SWZ, kFromRow>(part, s, in, peak);
+        fft_stage_of<MAXR, false, SWZ, kFromRow>(part, s, in, peak);
         part_sync();
     }
     if (pl.bluestein) {
-        fft_turn_of<SWZ>(part);
+        fft_turn_of<MAXR, SWZ>(part);
         part_sync();
         for (s = last - 1; s > 0; --s) {
-            fft_stage_of<true, SWZ, kFromRow>(part, s, in, peak);
+            fft_stage_of<MAXR, true, SWZ, kFromRow>(part, s, in, peak);
             part_sync();
         }
         __syncthreads();
         if (last > 0) {
-            fft_stage_of<true, SWZ, kToPeak>(whole, 0, in, peak);
+            fft_stage_of<MAXR, true, SWZ, kToPeak>(whole, 0, in, peak);
         } else {
             for (uint32_t k = threadIdx.x; k < pl.L; k += blockDim.x) peak.see(row[slot<SWZ>(k)], k);
         }
     } else if (last >= 0) {
-        fft_stage_of<false, SWZ, kToPeak>(part, last, in, peak);
+        fft_stage_of<MAXR, false, SWZ, kToPeak>(part, last, in, peak);
     } else {  // one sample
         if (threadIdx.x == 0) peak.see(row[0], 0u);
     }
@@ -1218,19 +1262,23 @@ cudaError_t launch_fft_tunes(const FftTuneArgs &a, cudaStream_t s) {
     if (a.n == 0) return cudaSuccess;
     if (a.plan.M == 0 || a.plan.M > kFftMaxLen || a.plan.L == 0) return cudaErrorInvalidValue;
     const size_t smem = fft_tune_smem_bytes(a.plan);
-    auto kernel = a.plan.swizzle == 4   ? fft_tune_kernel<4>
-                  : a.plan.swizzle == 3 ? fft_tune_kernel<3>
-                                        : fft_tune_kernel<0>;
+    const bool long_row = a.plan.M >= kFftLongRow;
+    auto kernel = long_row ? (a.plan.swizzle == 4   ? fft_tune_kernel<16, 4>
+                              : a.plan.swizzle == 3 ? fft_tune_kernel<16, 3>
+                                                    : fft_tune_kernel<16, 0>)
+                           : (a.plan.swizzle == 3 ? fft_tune_kernel<8, 3> : fft_tune_kernel<8, 0>);
     if (smem > 40u * 1024u) {
         const cudaError_t e =
             cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
         if (e != cudaSuccess) return e;
     }
-    // About one radix-16 butterfly per thread and stage, whole warps in each
-    // group.
-    const uint32_t step = 32u * kFftGroups;
-    const uint32_t want = (a.plan.M / 16u + step - 1u) / step * step;
-    const int threads = int(std::min<uint32_t>(kFftThreadsMax, std::max(step, want)));
+    // About one butterfly of the largest radix per thread and stage; whole
+    // warps in each group of a long row.
+    const uint32_t step = long_row ? 32u * kFftGroups : 32u;
+    const uint32_t least = long_row ? step : 64u;
+    const uint32_t most = uint32_t(long_row ? kFftThreadsMax<16> : kFftThreadsMax<8>);
+    const uint32_t want = (a.plan.M / (long_row ? 16u : 8u) + step - 1u) / step * step;
+    const int threads = int(std::min(most, std::max(least, want)));
     int dev = 0, sms = 0, per_sm = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
