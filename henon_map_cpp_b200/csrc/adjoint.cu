@@ -239,8 +239,7 @@ __global__ void __launch_bounds__(kThreads, P == 1 ? 4 : 3) adjoint_inverse_kern
 #pragma unroll
     for (int j = 0; j < P; ++j) {
         loss[j] = 0.0;
-        // (the gradient call counts a point lost before the first turn as N)
-        lost_at[j] = GRAD || alive[j] ? N : 0u;
+        lost_at[j] = alive[j] ? N : 0u;
     }
     uint32_t next_ckpt = 0;  // turn of the next checkpoint store
     if (n_stages > 0) {
