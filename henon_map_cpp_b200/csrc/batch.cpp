@@ -266,6 +266,10 @@ hm_status hm_batch_create(size_t n_sets, const hm_batch_set *sets, hm_batch **ou
     for (size_t k = 0; k < n_sets; ++k) {
         const hm_batch_set &p = sets[k];
         b->kinds.emplace_back(p.modulation_kind ? p.modulation_kind : "sps");
+        if (const hm_status s = hm::check_modulation(b->kinds.back(), p.omega_0); s != HM_OK) {
+            delete b;
+            return s;
+        }
         const size_t turns = hm::table_turns(b->kinds.back(), p.n_turns, p.offset);
         specs.push_back({b->kinds.back(), uint32_t(turns), p.omega_x, p.omega_y, p.omega_0,
                          p.epsilon, p.offset, nullptr});

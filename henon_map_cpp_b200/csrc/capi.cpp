@@ -568,6 +568,7 @@ namespace {
 hm_status compute_tables(hm_tracker *t, uint32_t n_turns, double omega_x, double omega_y,
                          const char *kind, double omega_0, double epsilon, uint32_t offset) {
     if (!kind) return fail(HM_ERR_INVALID_ARG, "null modulation kind");
+    HM_TRY(hm::check_modulation(kind, omega_0));
     const size_t n = hm::table_turns(kind, n_turns, offset);
     std::vector<double> records(4 * n);
     HM_TRY(hm::turn_records({{kind, uint32_t(n), omega_x, omega_y, omega_0, epsilon, offset,

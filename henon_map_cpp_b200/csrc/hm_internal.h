@@ -45,6 +45,8 @@ bool cancel_requested();
 
 // ---- modulation (host, bit-identical to the reference) ---------------------
 
+// What modulation() refuses, before anything is allocated for its tables.
+hm_status check_modulation(const std::string &kind, double omega_0);
 hm_status modulation(const std::string &kind, uint32_t n_turns, double omega_x,
                      double omega_y, double omega_0, double epsilon,
                      uint32_t offset, std::vector<double> &wx,

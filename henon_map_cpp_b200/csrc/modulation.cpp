@@ -98,19 +98,26 @@ std::vector<double> basic_modulation(double tune, double omega, double epsilon,
     return out;
 }
 
+hm_status check_modulation(const std::string &kind, double omega_0) {
+    if (kind != "sps" && kind != "basic" && kind != "none" && kind != "gaussian" &&
+        kind != "uniform")
+        return fail(HM_ERR_UNKNOWN_MODULATION, "Unknown modulation kind");
+    if (kind == "basic" && std::isnan(omega_0))
+        return fail(HM_ERR_INVALID_ARG, "basic modulation needs a finite omega_0");
+    return ok();
+}
+
 hm_status modulation(const std::string &kind, uint32_t n_turns, double omega_x,
                      double omega_y, double omega_0, double epsilon,
                      uint32_t offset, std::vector<double> &wx,
                      std::vector<double> &wy) {
+    HM_TRY(check_modulation(kind, omega_0));
     const int32_t start = int32_t(offset);
     const int32_t end = int32_t(offset + n_turns);
     if (kind == "sps") {
         wx = sps_modulation(omega_x, epsilon, start, end);
         wy = sps_modulation(omega_y, epsilon, start, end);
     } else if (kind == "basic") {
-        if (std::isnan(omega_0))
-            return fail(HM_ERR_INVALID_ARG,
-                        "basic modulation needs a finite omega_0");
         wx = basic_modulation(omega_x, omega_0, epsilon, start, end);
         wy = basic_modulation(omega_y, omega_0, epsilon, start, end);
     } else if (kind == "none") {
@@ -118,7 +125,7 @@ hm_status modulation(const std::string &kind, uint32_t n_turns, double omega_x,
         // then reads past them; here the tables hold the constant angles.
         wx.assign(n_turns, omega_x);
         wy.assign(n_turns, omega_y);
-    } else if (kind == "gaussian" || kind == "uniform") {
+    } else {  // gaussian, uniform
         // Random tunes drawn per turn (src/modulation.cpp:62-99): angle =
         // 2*pi*sample with sample ~ N(omega, eps) or U(omega, eps).
         std::random_device rd;
@@ -135,8 +142,6 @@ hm_status modulation(const std::string &kind, uint32_t n_turns, double omega_x,
         };
         draw(omega_x, wx);
         draw(omega_y, wy);
-    } else {
-        return fail(HM_ERR_UNKNOWN_MODULATION, "Unknown modulation kind");
     }
     return ok();
 }
