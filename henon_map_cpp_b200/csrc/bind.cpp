@@ -14,6 +14,7 @@
 #include <cmath>
 #include <cstring>
 #include <limits>
+#include <memory>
 #include <stdexcept>
 #include <string>
 #include <vector>
@@ -84,10 +85,21 @@ double nan_std(const double *v, size_t n) {
 }
 
 // An ndarray itself: subclasses (masked arrays among them) may read their
-// elements otherwise, so a constructor from arrays leaves them, as all that
-// it does not take, to the one from lists (reference_cast_error).
-bool plain_array(const py::array &a) {
+// elements otherwise, so they are taken as lists are.
+bool plain_array(const py::handle &a) {
     return py::type::of(a).is(py::module_::import("numpy").attr("ndarray"));
+}
+
+// A constructor's argument as its C++ type, with the conversions of a function
+// that has no other overload; what does not convert is a TypeError of the
+// constructor.  (As overloads of their own, arrays and lists would be tried
+// without conversions first, which takes a third longer for lists of numpy
+// floats.)
+template <class T>
+T argument(const py::object &o) {
+    py::detail::make_caster<T> caster;
+    if (!caster.load(o, true)) throw py::reference_cast_error();
+    return py::detail::cast_op<T &&>(std::move(caster));
 }
 
 // ---- particles_4d_gpu --------------------------------------------------------------
@@ -100,7 +112,7 @@ struct Particles {
             throw py::value_error("x, px, y, py must have the same length");
         check(hm_particles_create(x.data(), px.data(), y.data(), py.data(), x.size(), &h));
     }
-    // The same from arrays of doubles (below): no list of Python floats.
+    // The same from one-dimensional arrays of doubles: no list of floats.
     using Array = py::array_t<double, 0>;
     Particles(const Array &x, const Array &px, const Array &y, const Array &py_) {
         const Array *in[4] = {&x, &px, &y, &py_};
@@ -108,7 +120,6 @@ struct Particles {
         const double *data[4];
         std::vector<double> strided[4];
         for (int f = 0; f < 4; ++f) {
-            if (!plain_array(*in[f]) || in[f]->ndim() != 1) throw py::reference_cast_error();
             if (size_t(in[f]->size()) != n)
                 throw py::value_error("x, px, y, py must have the same length");
             data[f] = in[f]->data();
@@ -207,8 +218,6 @@ struct Vectors {
     }
     using Array = py::array_t<double, py::array::c_style>;
     explicit Vectors(const Array &rv) {
-        if (!plain_array(rv) || rv.ndim() != 2 || rv.shape(1) != 4)
-            throw py::reference_cast_error();
         n = size_t(rv.shape(0));
         check(hm_vectors_create(rv.data(), n, &h));
     }
@@ -395,14 +404,24 @@ class storage_4d(_CpuClassNotProvided):
     // ---- particles_4d_gpu ----------------------------------------------------------
     // Arrays of float64 (any stride) are taken as they are: 1.9 ms instead of
     // 156 ms for 2^20 particles.  Everything else that converts to a list of
-    // floats takes the second constructor.
+    // floats is converted.
     py::class_<Particles>(m, "particles_4d_gpu")
-        .def(py::init<const Particles::Array &, const Particles::Array &, const Particles::Array &,
-                      const Particles::Array &>(),
-             py::arg("x").noconvert(), py::arg("px").noconvert(), py::arg("y").noconvert(),
-             py::arg("py").noconvert())
-        .def(py::init<const std::vector<double> &, const std::vector<double> &,
-                      const std::vector<double> &, const std::vector<double> &>(),
+        .def(py::init([](const py::object &x, const py::object &px, const py::object &y,
+                         const py::object &py_) {
+                 using Array = Particles::Array;
+                 const py::object *const in[4] = {&x, &px, &y, &py_};
+                 bool arrays = true;
+                 for (const py::object *o : in)
+                     arrays = arrays && py::isinstance<Array>(*o) && plain_array(*o) &&
+                              py::reinterpret_borrow<py::array>(*o).ndim() == 1;
+                 if (arrays)
+                     return std::make_unique<Particles>(
+                         py::reinterpret_borrow<Array>(x), py::reinterpret_borrow<Array>(px),
+                         py::reinterpret_borrow<Array>(y), py::reinterpret_borrow<Array>(py_));
+                 using List = std::vector<double>;
+                 return std::make_unique<Particles>(argument<List>(x), argument<List>(px),
+                                                    argument<List>(y), argument<List>(py_));
+             }),
              py::arg("x"), py::arg("px"), py::arg("y"), py::arg("py"))
         .def("reset", [](Particles &p) { check(hm_particles_reset(p.h)); })
         // Key of the reproducible random kicks of track(kick_module=...);
@@ -672,8 +691,13 @@ class storage_4d(_CpuClassNotProvided):
         }, py::arg("vector"));
 
     py::class_<Vectors>(m, "vector_4d_gpu")
-        .def(py::init<const Vectors::Array &>(), py::arg("rv").noconvert())
-        .def(py::init<const std::vector<std::vector<double>> &>())
+        .def(py::init([](const py::object &rv) {
+            if (py::isinstance<Vectors::Array>(rv) && plain_array(rv)) {
+                const auto a = py::reinterpret_borrow<Vectors::Array>(rv);
+                if (a.ndim() == 2 && a.shape(1) == 4) return std::make_unique<Vectors>(a);
+            }
+            return std::make_unique<Vectors>(argument<std::vector<std::vector<double>>>(rv));
+        }))
         .def("set_vectors", [](Vectors &v, py::array_t<double, py::array::c_style |
                                                                  py::array::forcecast> a) {
             if (a.size() == 4 && a.ndim() == 1) {
