@@ -35,7 +35,8 @@ constexpr size_t kPiece = 1024;
 
 template <class F> void parallel_pieces(size_t n, F body) {
     const size_t pieces = (n + kPiece - 1) / kPiece;
-    const size_t hw = std::max<size_t>(1, std::thread::hardware_concurrency());
+    // (asked once: it reads a file, 2 us of a table of one turn's 10)
+    static const size_t hw = std::max<size_t>(1, std::thread::hardware_concurrency());
     std::atomic<size_t> next{0};
     auto work = [&] {
         for (size_t q; (q = next.fetch_add(1)) < pieces;)
