@@ -150,21 +150,24 @@ __device__ __forceinline__ Turn staged_record(const double *rec, uint32_t kn, ui
 // second turn is 1.35 for barrier 10, 0.50 for 2 and 0.31 for 1, that of every
 // turn half the barrier): after kVainRedos blocks of a stage that were redone
 // for nothing the warp looks, or tests, that way for the rest of the stage.
-// One such block is more often an orbit on its way out.  ms for 10^4 turns,
-// with per-turn looks in runs of 32, with blocks that were all retested, now:
+// A single one is more often an orbit on its way out: with 2 in place of 4 the
+// loss-heavy start of a scan took 8 % more with two particles per thread
+// (1024^2 points on [0, 0.6]^2, 3,000 turns, mu = 0.2: 6.7 and 6.3 ms), and a
+// small barrier 2-10 % less.  ms for 10^4 turns, with per-turn looks in runs of
+// 32, with blocks that were all retested, now:
 //     barrier             0.8    1      2      3      10
 //     90,000 particles    4.16   4.52   4.07   4.05   2.02
 //       (mu = 0.2)        5.75   5.61   4.73   4.24   1.87
-//                         3.10   3.11   2.19   2.03   1.82
+//                         3.31   3.31   2.24   2.16   1.80
 //     3,600 particles     2.22   1.94   1.74   1.75   0.47
 //       (mu = 0)          2.42   2.12   1.76   0.56   0.33
-//                         1.91   1.51   0.40   0.35   0.33
+//                         1.95   1.64   0.45   0.36   0.33
 enum class Look {
     kPairs,  // at every second turn
     kEvery,  // at every turn
     kTest,   // the test itself
 };
-constexpr uint32_t kVainRedos = 2;
+constexpr uint32_t kVainRedos = 4;
 
 // Returns false when a copy did not land within the bounded wait (the
 // chunk's results are then invalid and c.fault is set).
