@@ -26,8 +26,10 @@ struct TrackConfig {
     int threads = 128;
     // One particle per thread: a redo (track.cu turns_staged) repeats the
     // turns of 32 particles instead of 64, and short lists balance better.
-    // 1024^2 grid on [0, 0.6]^2, mu = 0.2, 2e4 turns: 28.0 ms against 29.6
-    // with two; fast arithmetic, 701^2, mu = 0: 7.45 against 7.69.
+    // 1024^2 grid on [0, 0.6]^2, epsilon = 64, kernel ms with one and two:
+    //               mu = 0, 2e4 turns   1e5           mu = 0.2, 2e4   1e5
+    //     exact     16.3  17.1          66.0  67.8    26.7  29.0      107.1  112.2
+    //     fast      14.1  14.4          57.1  56.9    19.0  19.5       76.2   76.7
     int per_thread = 1;
     uint32_t chunk0 = 512;      // turns of the first chunk
     uint32_t chunk_max = 16384; // chunk length cap (chunks double up to it)

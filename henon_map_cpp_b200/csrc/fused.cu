@@ -476,8 +476,12 @@ cudaError_t launch4(const FusedArgs &a, cudaStream_t s) {
     return cudaGetLastError();
 }
 
-// Lyapunov and tune windows open per turn from which the y plane's tunes are
-// better off with the matrix work: between the 5.6 and the 10.8 measured above.
+// Lyapunov and tune windows open per turn above which the y plane's tunes are
+// better off with the matrix work at every size: with windows of one length,
+// open throughout, the split takes 0.95-1.00 of the time at 2 open windows,
+// 0.92-0.96 at 6, 0.89-0.93 at 8, 0.90-0.92 at 12 and 0.79-0.83 at 26 (500 to
+// 150,000 particles); with windows that close one after the other it was
+// slower at 5.6 and faster at 10.8 open on average (above, both kinds).
 constexpr double kPlanesOpen = 8.0;
 
 template <bool OCT>

@@ -404,7 +404,7 @@ __device__ __forceinline__ bool small_or(uint32_t ored, const Barrier &b) {
 
 // The largest |high word| of a and b and of the running maximum m, taken on
 // the words read as single floats: for sign-free patterns both orders agree,
-// and a pattern at or above 0x7f800000 (a coordinate of 2^1016 or more, an
+// and a pattern at or above 0x7f800000 (a coordinate of 2^1017 or more, an
 // infinity or a NaN) gives infinity or, with .NaN, a NaN, whose pattern is
 // above every bound.  One instruction for two coordinates.
 __device__ __forceinline__ float hi_max(float m, double a, double b) {

@@ -90,9 +90,10 @@ int hm_version(void);
 /* Number of CUDA devices visible (0 when none); never fails. */
 int hm_device_count(void);
 
-/* Called between turn chunks of every long operation; a non-zero return
- * stops the operation with HM_ERR_CANCELLED after the state has been made
- * consistent (replaces check_keyboard_interrupt, src/henon.cu:7-15). */
+/* Called between turn chunks of every long operation (hm_track: of 512
+ * turns, doubling to 16384); a non-zero return stops the operation with
+ * HM_ERR_CANCELLED after the state has been made consistent (replaces
+ * check_keyboard_interrupt, src/henon.cu:7-15). */
 typedef int (*hm_cancel_fn)(void *ctx);
 hm_status hm_set_cancel_callback(hm_cancel_fn fn, void *ctx);
 
@@ -538,13 +539,14 @@ hm_status hm_storage_tunes(const hm_storage *s, const uint32_t *from,
  * reconstruction error bounded to one segment).  mode 1 gives grad_ic by
  * forward-mode tangent-map propagation (an independent J^T v) and, when
  * grad_theta is not NULL, grad_theta by forward propagation of the state's
- * derivatives with respect to theta alongside it; mode 2 the loss only.
- * Derivatives need an "sps" or "basic" modulation.  Synchronous. */
+ * derivatives with respect to theta alongside it; mode 2 the loss only (mode
+ * 3's forward sweep).  steps[i] is the turns the particle survived: n_turns,
+ * or less when lost (0 when it starts as NaN).  Derivatives need an "sps" or "basic" modulation.  Synchronous. */
 size_t hm_adjoint_workspace_bytes(size_t n, uint32_t n_turns,
                                   uint32_t checkpoint_every);
-/* Most particles per thread of mode 3's kernel (1 or 2; default 2, which a
- * call uses where its size makes it the faster one).  Process-wide; results
- * do not depend on it. */
+/* Most particles per thread of the kernel of modes 2 and 3 (1 or 2; default
+ * 2, which a call uses where its size makes it the faster one).
+ * Process-wide; results do not depend on it. */
 hm_status hm_set_adjoint_config(int per_thread);
 hm_status hm_get_adjoint_config(int *per_thread);
 hm_status hm_adjoint(const hm_tracker *t, const double *x0, const double *px0,
