@@ -604,7 +604,9 @@ hm_status track_indicators(hm_tracker *t, hm_particles *p, uint32_t n_turns, dou
     // structured_multiply after the last turn.
     const bool tangent = (s.matrix || s.vectors) && !s.jacobian_of_turn;
     if (inverse) {
-        if (n_turns > p->global_steps || n_turns > p->live_step)
+        // (the records read are those below the particles' own steps)
+        if (n_turns > p->global_steps || n_turns > p->live_step ||
+            p->live_step > t->allowed_steps)
             return fail(HM_ERR_BUDGET, "The number of turns is too large.");
     } else if (uint64_t(n_turns) + p->global_steps + (tangent ? 1 : 0) > t->allowed_steps) {
         return fail(HM_ERR_BUDGET, "The number of turns is too large.");

@@ -327,7 +327,9 @@ hm_status hm_tracker_orbit_tunes(hm_tracker *t, hm_particles *p, uint32_t n_turn
                                  int remove_mean, double *birkhoff_out, double *fft_out) {
     if (!t || !p) return fail(HM_ERR_INVALID_ARG, "null tracker or particles");
     if (inverse) {
-        if (n_turns > p->global_steps || n_turns > p->live_step)
+        // (the records read are those below the particles' own steps)
+        if (n_turns > p->global_steps || n_turns > p->live_step ||
+            p->live_step > t->allowed_steps)
             return fail(HM_ERR_BUDGET, "The number of turns is too large.");
     } else if (uint64_t(n_turns) + p->global_steps > t->allowed_steps) {
         return fail(HM_ERR_BUDGET, "The number of turns is too large.");
