@@ -772,9 +772,10 @@ hm_status hm_tracker_megno(hm_tracker *t, hm_particles *p, uint32_t n_turns, dou
                 for (size_t j = 0; j < n_samples; ++j)
                     host_out[i * n_samples + j] = snap[j * n + i];
     }
+    const std::string why = hm_last_error();  // (cleared by the destructors)
     hm_megno_destroy(g);
     hm_matrices_destroy(M);
-    return st;
+    return st == HM_OK ? ok() : fail(st, why);
 }
 
 hm_status hm_storage_device_ptr(const hm_storage *h, hm_field field, const double **out) {

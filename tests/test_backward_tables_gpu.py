@@ -28,7 +28,7 @@ def test_shorter_table_is_refused(gpu, turns):
         short.track(p, 5, 0.0, 10.0, NAN, True)
     with pytest.raises(C.HMError, match=message):
         C.tracker_orbit_tunes(short, p, 5, 0.0, 10.0, [], [], False, False, NAN, True)
-    with pytest.raises(C.HMError):
+    with pytest.raises(C.HMError, match=message):
         C.call("hm_tracker_megno", short.h, p.h, 5, 0.0, 10.0, NAN, 1,
                samples.ctypes.data_as(ctypes.POINTER(ctypes.c_uint64)), 1, C.dptr(out))
     assert p.global_steps == 100
