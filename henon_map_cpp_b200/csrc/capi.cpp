@@ -575,8 +575,27 @@ hm_status compute_tables(hm_tracker *t, uint32_t n_turns, double omega_x, double
     std::vector<double> records(4 * n);
     HM_TRY(hm::turn_records({{kind, uint32_t(n), omega_x, omega_y, omega_0, epsilon, offset,
                               records.data()}}));
+    // The tables there are stay until the new ones are on the device.  Where
+    // those fit only in their place they go first, and should the new ones not
+    // come through then, the tracker has none.
+    hm::DeviceBuffer table;
+    hm_status up = hm::upload(table, records);
+    if (up == HM_ERR_OOM && t->table.ptr) {
+        const std::string why = hm_last_error();
+        size_t free_b = 0;
+        if (hm::device_free_bytes(&free_b) == HM_OK &&
+            free_b + t->table.bytes >= records.size() * sizeof(double)) {
+            t->table.release();
+            t->records.clear();
+            t->allowed_steps = 0;
+            up = hm::upload(table, records);
+        } else {
+            up = fail(up, why);
+        }
+    }
+    HM_TRY(up);
+    t->table = std::move(table);
     t->records = std::move(records);
-    HM_TRY(hm::upload(t->table, t->records));
     t->allowed_steps = n;
     {
         // the adjoint's ripple follows the modulation
